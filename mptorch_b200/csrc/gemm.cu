@@ -2,7 +2,7 @@
 // statistics, problem set-up.  The kernel lives in gemm_kernel.cuh, its instantiations in gemm_*.cu.
 #include <cmath>
 
-#include "gemm_kernel.cuh"
+#include "gemm16_kernel.cuh"
 
 namespace mpt {
 namespace {
@@ -122,6 +122,13 @@ int run_mm(const float* a, const float* b, float* c, int64_t batch, int M, int N
     // (2^33 MACs, about 2 ms) get it; shorter ones keep the exact path inside mm_kernel for such entries.
     const bool defer = algo != ALGO_SR && p.stats != nullptr && (double)batch * M * N * K >= 8589934592.0;
     p.defer_exact = defer ? 1 : 0;
+    p.vec = vec ? 1 : 0;
+    // formats whose sums fit a 16-bit register: the same bits from a third to a half of the arithmetic (gemm16_kernel.cuh)
+    p.kind16 = (p.stats != nullptr && algo != ALGO_SR && use_packed()) ? kind16_of(fadd, fmul, fma) : -1;
+    if (p.kind16 >= 0) {
+        const int rc = small ? launch_mm16_small(algo, p, batch, st) : launch_mm16(algo, p, batch, st);
+        return (rc || !defer) ? rc : launch_mm_exact(algo, fma, p, batch, st);
+    }
     if (nosub && p.stats != nullptr) {
         const int rc = launch_mm_nosub(algo, fma, p, batch, vec, st);
         return (rc || !defer) ? rc : launch_mm_exact(algo, fma, p, batch, st);
@@ -167,6 +174,7 @@ int run_conv(const float* x, const float* wt, float* y, int n_img, int c_in, int
     const bool fast_candidate = (nosub || (fast_rn_supported(fadd) && (fma || fast_rn_supported(fmul)))) && workspace != nullptr &&
                                 workspace_bytes >= sizeof(MmStats) && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0 && K64 > 0;
     p.nosub = (nosub && fast_candidate) ? 1 : 0;
+    p.kind16 = (fast_candidate && use_packed()) ? kind16_of(fadd, p.fmul, fma) : -1;
     if (K64 == 0) {
         cudaError_t e = cudaMemsetAsync(y, 0, sizeof(float) * (size_t)n_img * c_out * OH * OW, st);
         if (e != cudaSuccess) { set_error("float_conv2d: cudaMemsetAsync: %s", cudaGetErrorString(e)); return MPT_ERR_CUDA; }
@@ -189,7 +197,7 @@ int run_conv(const float* x, const float* wt, float* y, int n_img, int c_in, int
         p.a = x + (int64_t)g * cg * H * W;
         p.b = wt + (int64_t)g * K64 * og;
         p.c = y + (int64_t)g * og * OH * OW;
-        const int rc = launch_conv_any(algo, fma, p, st);
+        const int rc = p.kind16 >= 0 ? launch_conv16(algo, p, st) : launch_conv_any(algo, fma, p, st);
         if (rc) return rc;
     }
     return MPT_OK;
@@ -229,6 +237,7 @@ int run_conv_wgrad(const float* gout, const float* x, float* gw, int n_img, int 
     const bool fast_candidate = (nosub || (fast_rn_supported(fadd) && (fma || fast_rn_supported(fmul)))) && workspace != nullptr &&
                                 workspace_bytes >= sizeof(MmStats) && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
     p.nosub = (nosub && fast_candidate) ? 1 : 0;
+    p.kind16 = (fast_candidate && use_packed()) ? kind16_of(fadd, p.fmul, fma) : -1;
     if (fast_candidate) {
         MmStats* s = static_cast<MmStats*>(workspace);
         stats_init_kernel<<<1, 256, 0, st>>>(s, 1);
@@ -248,7 +257,8 @@ int run_conv_wgrad(const float* gout, const float* x, float* gw, int n_img, int 
         // fewer 128-row tiles than SMs: the 16-row instantiation spreads the same outputs over eight times the CTAs
         const int64_t big_tiles = (((int64_t)p.M + BM - 1) / BM) * (((int64_t)p.N + BN - 1) / BN);
         const bool small = big_tiles < sm_count() && ((int64_t)p.M + kSmallTileRows - 1) / kSmallTileRows <= 65535;
-        const int rc = small ? launch_conv_wgrad_small_any(algo, fma, p, st) : launch_conv_wgrad_any(algo, fma, p, st);
+        const int rc = p.kind16 >= 0 ? (small ? launch_conv16_wgrad_small(algo, p, st) : launch_conv16_wgrad(algo, p, st))
+                     : small ? launch_conv_wgrad_small_any(algo, fma, p, st) : launch_conv_wgrad_any(algo, fma, p, st);
         if (rc) return rc;
     }
     return MPT_OK;
@@ -297,6 +307,14 @@ int static_scratch_address(void** out) {
 }
 
 }  // namespace
+
+int launch_mm16_seq(const MmParams& p, int64_t batch, cudaStream_t st);      // gemm16_seq.cu, gemm16_tile8.cu, gemm16_kahan.cu
+int launch_mm16_tile8(const MmParams& p, int64_t batch, cudaStream_t st);
+int launch_mm16_kahan(const MmParams& p, int64_t batch, cudaStream_t st);
+int launch_mm16(int algo, const MmParams& p, int64_t batch, cudaStream_t st) {
+    return algo == ALGO_SEQ ? launch_mm16_seq(p, batch, st) : algo == ALGO_TILE8 ? launch_mm16_tile8(p, batch, st) : launch_mm16_kahan(p, batch, st);
+}
+
 }  // namespace mpt
 
 using namespace mpt;

@@ -115,6 +115,8 @@ struct MmParams {
     // which is shaped for the exact casters; mm_kernel returns at once for it, exact_mm_kernel for every other entry.
     int defer_exact = 0;
     int nosub = 0;               // the formats have no subnormals and the launch is of the NOSUB instantiation
+    int vec = 0;                 // operands admit 16-byte copies (mm16_kernel, which has one form for both)
+    int kind16 = -1;             // format pair of mm16_kernel (gemm16_kernel.cuh), -1: none
 };
 enum { MM_FROM_C = 1, MM_MORE = 2 };
 
@@ -712,6 +714,104 @@ __device__ __forceinline__ FastPlan make_plan(const MmParams& p, int64_t batch) 
     return plan;
 }
 
+// CTAs are launched x-fastest; walking the output in bands of kGroupM row tiles (all column tiles of a band before
+// the next band) keeps the A rows and B columns that concurrently resident CTAs share inside L2, so the operands
+// are read from HBM a few times instead of once per row of tiles.
+__device__ __forceinline__ void banded_tile(int& tile_m, int& tile_n) {
+    constexpr int kGroupM = 8;
+    // 64-bit: gridDim.x * gridDim.y can pass 2^31 for a very wide N
+    const uint64_t pid = (uint64_t)blockIdx.y * gridDim.x + blockIdx.x;
+    const uint64_t per_band = (uint64_t)kGroupM * gridDim.x;
+    const int band = (int)(pid / per_band);
+    const uint64_t in_band = pid - (uint64_t)band * per_band;
+    const int first_m = band * kGroupM;
+    const int rows_here = min((int)gridDim.y - first_m, kGroupM);
+    tile_n = (int)(in_band / (unsigned)rows_here);
+    tile_m = first_m + (int)(in_band - (uint64_t)tile_n * rows_here);
+}
+
+// CONV_FWD: image offset and top-left input coordinate of the tile's BM output positions.
+__device__ __forceinline__ void fill_conv_rows(const MmParams& p, ConvRow* crow, int m0, int tid) {
+    if (tid >= BM) return;
+    const int gm = m0 + tid;
+    ConvRow r;
+    if (gm < p.M) {
+        const int L = p.cv.OH * p.cv.OW;
+        const int img = gm / L, l = gm - img * L;
+        const int oh = l / p.cv.OW, ow = l - oh * p.cv.OW;
+        r.base = (int64_t)img * p.cv.x_image_stride;
+        r.ih0 = oh * p.cv.sh - p.cv.ph;
+        r.iw0 = ow * p.cv.sw - p.cv.pw;
+    } else {
+        r.base = 0; r.ih0 = -(1 << 30); r.iw0 = -(1 << 30);      // fails every bounds check: zero rows
+    }
+    crow[tid] = r;
+}
+
+// The thread's outputs as C holds them (zero outside the matrix).
+__device__ __forceinline__ void load_c(const MmParams& p, const float* C, int m0, int n0, int ty, int tx, float (&v)[TM][TN]) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int gm = m0 + ty + 16 * i;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int gn = n0 + tx * 4 + j;
+            v[i][j] = (gm < p.M && gn < p.N) ? C[(int64_t)gm * p.N + gn] : 0.0f;
+        }
+    }
+}
+
+// Eight compensated steps from slab row kbase on the whole-domain casters; aux = compensation terms.
+template <bool FMA>
+__device__ __forceinline__ void kahan_exact_group(float (&acc)[TM][TN], float (&aux)[TM][TN], const float* as, const float* bs,
+                                                  int kbase, int ty, int tx, const MmParams& p) {
+#pragma unroll 1
+    for (int k = kbase; k < kbase + 8; ++k) {
+        const float4 bv4 = *reinterpret_cast<const float4*>(bs + k * BN + tx * 4);
+        const float bvv[4] = {bv4.x, bv4.y, bv4.z, bv4.w};
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const float a = as[(ty + 16 * i) * AS_LD + k];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) kahan_exact<FMA>(acc[i][j], aux[i][j], a, bvv[j], p);
+        }
+    }
+}
+
+template <int CONV>
+__device__ __forceinline__ void store_tile(const MmParams& p, float* C, int m0, int n0, int ty, int tx, bool vec, const float (&v)[TM][TN]) {
+    if (CONV == CONV_FWD) {     // C[m][n] goes to y[image][n][oh][ow]: consecutive m are consecutive addresses
+        const int L = p.cv.OH * p.cv.OW;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int gm = m0 + ty + 16 * i;
+            if (gm >= p.M) continue;
+            const int img = gm / L, l = gm - img * L;
+            float* dst = C + (int64_t)img * p.cv.y_image_stride + l;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int gn = n0 + tx * 4 + j;
+                if (gn < p.N) dst[(int64_t)gn * L] = v[i][j];
+            }
+        }
+        return;
+    }
+    const bool vec_store = vec && ((reinterpret_cast<uintptr_t>(C) & 15u) == 0);
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int gm = m0 + ty + 16 * i;
+        if (gm >= p.M) continue;
+        const int gn = n0 + tx * 4;
+        float* dst = C + (int64_t)gm * p.N + gn;
+        if (vec_store && gn + 3 < p.N) *reinterpret_cast<float4*>(dst) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+        else {
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+                if (gn + j < p.N) dst[j] = v[i][j];
+        }
+    }
+}
+
 template <int ALGO, bool FMA, bool VEC, bool PACKED, bool ADDG, int CONV = CONV_NONE, int MINB = MPT_MM_MIN_CTAS, bool NOSUB = false>
 __global__ void __launch_bounds__(THREADS, MINB) mm_kernel(const __grid_constant__ MmParams p) {
     extern __shared__ __align__(16) float smem[];
@@ -721,22 +821,8 @@ __global__ void __launch_bounds__(THREADS, MINB) mm_kernel(const __grid_constant
 
     const int tid = threadIdx.x;
     const int ty = tid >> 4, tx = tid & 15;
-    // CTAs are launched x-fastest; walking the output in bands of kGroupM row tiles (all column tiles of a band before
-    // the next band) keeps the A rows and B columns that concurrently resident CTAs share inside L2, so the operands
-    // are read from HBM a few times instead of once per row of tiles.
     int tile_m, tile_n;
-    {
-        constexpr int kGroupM = 8;
-        // 64-bit: gridDim.x * gridDim.y can pass 2^31 for a very wide N
-        const uint64_t pid = (uint64_t)blockIdx.y * gridDim.x + blockIdx.x;
-        const uint64_t per_band = (uint64_t)kGroupM * gridDim.x;
-        const int band = (int)(pid / per_band);
-        const uint64_t in_band = pid - (uint64_t)band * per_band;
-        const int first_m = band * kGroupM;
-        const int rows_here = min((int)gridDim.y - first_m, kGroupM);
-        tile_n = (int)(in_band / (unsigned)rows_here);
-        tile_m = first_m + (int)(in_band - (uint64_t)tile_n * rows_here);
-    }
+    banded_tile(tile_m, tile_n);
     const int m0 = tile_m * BM, n0 = tile_n * BN;
     const int64_t batch = blockIdx.z;
     const float* A = p.a + batch * p.stride_a;
@@ -752,21 +838,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm_kernel(const __grid_constant
     if (CONV == CONV_NONE && p.defer_exact && !plan.ok) return;
 
     if (CONV == CONV_FWD) {
-        if (tid < BM) {
-            const int gm = m0 + tid;
-            ConvRow r;
-            if (gm < p.M) {
-                const int L = p.cv.OH * p.cv.OW;
-                const int img = gm / L, l = gm - img * L;
-                const int oh = l / p.cv.OW, ow = l - oh * p.cv.OW;
-                r.base = (int64_t)img * p.cv.x_image_stride;
-                r.ih0 = oh * p.cv.sh - p.cv.ph;
-                r.iw0 = ow * p.cv.sw - p.cv.pw;
-            } else {
-                r.base = 0; r.ih0 = -(1 << 30); r.iw0 = -(1 << 30);      // fails every bounds check: zero rows
-            }
-            crow[tid] = r;
-        }
+        fill_conv_rows(p, crow, m0, tid);
         __syncthreads();
     }
 
@@ -777,16 +849,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm_kernel(const __grid_constant
 #pragma unroll
         for (int j = 0; j < TN; ++j) { acc[i][j] = 0.0f; aux[i][j] = 0.0f; }
     if (CONV == CONV_NONE && (ALGO == ALGO_SEQ || ALGO == ALGO_TILE8) && (p.resume & MM_FROM_C)) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            const int gm = m0 + ty + 16 * i;
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const int gn = n0 + tx * 4 + j;
-                const float v = (gm < p.M && gn < p.N) ? C[(int64_t)gm * p.N + gn] : 0.0f;
-                if (ALGO == ALGO_TILE8) aux[i][j] = v; else acc[i][j] = v;
-            }
-        }
+        if (ALGO == ALGO_TILE8) load_c(p, C, m0, n0, ty, tx, aux); else load_c(p, C, m0, n0, ty, tx, acc);
     }
 
 #pragma unroll
@@ -855,17 +918,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm_kernel(const __grid_constant
                 if (PACKED && plan.ok && absmax_of(acc) < plan.acc_limit && absmax_of(aux) < plan.acc_limit) {
                     kahan_group_fast<FMA, ADDG>(acc, aux, as, bs, g * 8, ty, tx, p);
                 } else {
-#pragma unroll 1
-                    for (int k = g * 8; k < g * 8 + 8; ++k) {
-                        const float4 bv4 = *reinterpret_cast<const float4*>(bs + k * BN + tx * 4);
-                        const float bvv[4] = {bv4.x, bv4.y, bv4.z, bv4.w};
-#pragma unroll
-                        for (int i = 0; i < TM; ++i) {
-                            const float a = as[(ty + 16 * i) * AS_LD + k];
-#pragma unroll
-                            for (int j = 0; j < TN; ++j) kahan_exact<FMA>(acc[i][j], aux[i][j], a, bvv[j], p);
-                        }
-                    }
+                    kahan_exact_group<FMA>(acc, aux, as, bs, g * 8, ty, tx, p);
                 }
             }
         } else {   // ALGO_SR
@@ -889,39 +942,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm_kernel(const __grid_constant
     }
     cp_async_wait<0>();
 
-    // epilogue
-    if (CONV == CONV_FWD) {     // C[m][n] goes to y[image][n][oh][ow]: consecutive m are consecutive addresses
-        const int L = p.cv.OH * p.cv.OW;
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            const int gm = m0 + ty + 16 * i;
-            if (gm >= p.M) continue;
-            const int img = gm / L, l = gm - img * L;
-            const float* r = (ALGO == ALGO_TILE8) ? aux[i] : acc[i];
-            float* dst = C + (int64_t)img * p.cv.y_image_stride + l;
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const int gn = n0 + tx * 4 + j;
-                if (gn < p.N) dst[(int64_t)gn * L] = r[j];
-            }
-        }
-        return;
-    }
-    const bool vec_store = VEC && ((reinterpret_cast<uintptr_t>(C) & 15u) == 0);
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty + 16 * i;
-        if (gm >= p.M) continue;
-        const float* r = (ALGO == ALGO_TILE8) ? aux[i] : acc[i];
-        const int gn = n0 + tx * 4;
-        float* dst = C + (int64_t)gm * p.N + gn;
-        if (vec_store && gn + 3 < p.N) *reinterpret_cast<float4*>(dst) = make_float4(r[0], r[1], r[2], r[3]);
-        else {
-#pragma unroll
-            for (int j = 0; j < TN; ++j)
-                if (gn + j < p.N) dst[j] = r[j];
-        }
-    }
+    if (ALGO == ALGO_TILE8) store_tile<CONV>(p, C, m0, n0, ty, tx, VEC, aux); else store_tile<CONV>(p, C, m0, n0, ty, tx, VEC, acc);
 }
 
 // The packed fp32x2 fast path is the default; MPT_MM_SCALAR=1 in the environment selects the scalar
@@ -1013,6 +1034,12 @@ int launch_conv_wgrad_small_any(int algo, bool fma, const MmParams& p, cudaStrea
 int launch_mm_small(int algo, bool fma, const MmParams& p, int64_t batch, bool vec, cudaStream_t st);   // ALGO_SEQ / ALGO_TILE8
 int launch_mm_exact(int algo, bool fma, const MmParams& p, int64_t batch, cudaStream_t st);             // all but ALGO_SR
 int launch_mm_nosub(int algo, bool fma, const MmParams& p, int64_t batch, bool vec, cudaStream_t st);  // ALGO_SEQ / ALGO_TILE8
+// The same products on 16-bit running sums (gemm16_kernel.cuh), for p.kind16 >= 0.
+int launch_mm16(int algo, const MmParams& p, int64_t batch, cudaStream_t st);                            // all but ALGO_SR
+int launch_mm16_small(int algo, const MmParams& p, int64_t batch, cudaStream_t st);                      // ALGO_SEQ / ALGO_TILE8
+int launch_conv16(int algo, const MmParams& p, cudaStream_t st);
+int launch_conv16_wgrad(int algo, const MmParams& p, cudaStream_t st);
+int launch_conv16_wgrad_small(int algo, const MmParams& p, cudaStream_t st);
 constexpr int kSmallTileRows = 16;      // tile height of the instantiation behind launch_conv_wgrad_small_any
 
 }  // namespace mpt
