@@ -45,6 +45,30 @@ KahanBounds kahan_bounds(int man) {
     return KahanBounds{(top.v[0] + top.v[1]) * 1.001, top.v[2] * 1.001, top.v[3] * 1.001};
 }
 
+// Which tiles of the 16-bit kernel: 8 x 32 with one pair per thread (thin), 64 x 64 or 128 x 64?  A product takes the time of
+// the SM with the most tiles.  Measured for e4m3 products into e5m10 sums (clocks per K step and SM; the other formats scale
+// alike): n thin tiles 13 + 12 n, n tiles of 64 rows 122 n but never under 149, n of 128 rows 238 n.  256 x 256 x 4096: 94 us
+// thin, 310 and 490 otherwise; 768 x 768 x 1024: 140, 109, 156; 2048^2 x 512: 385, 239, 250.
+enum Tile16 { TILE16_THIN, TILE16_MID, TILE16_BIG };
+Tile16 pick_tile16(int M, int N, int64_t batch, bool thin_allowed) {
+    const int64_t sms = sm_count(), tn = ((int64_t)N + BN - 1) / BN;
+    const auto per_sm = [&](int64_t tiles) { return (double)((tiles + sms - 1) / sms); };
+    const double big = 238.0 * per_sm(((int64_t)M + BM - 1) / BM * tn * batch);
+    const int64_t rows_mid = ((int64_t)M + 63) / 64, rows_thin = ((int64_t)M + 7) / 8;
+    const double mid = rows_mid > 65535 ? 1e300 : fmax(149.0, 122.0 * per_sm(rows_mid * tn * batch));
+    const double thin = !thin_allowed || rows_thin > 65535 ? 1e300 : 13.0 + 12.0 * per_sm(rows_thin * (((int64_t)N + 31) / 32) * batch);
+    return thin < mid && thin < big ? TILE16_THIN : mid < big ? TILE16_MID : TILE16_BIG;
+}
+// The same for the gathered weight gradient (thin or 128 x 64): 25 + 23 n against 320 n.  64 channels at 64 x 56 x 56: 4.9 ms
+// thin, 30.7 otherwise; 256 channels at 16 x 14 x 14: 0.58 and 0.53.
+bool thin_wgrad16(int M, int N) {
+    const int64_t sms = sm_count();
+    const auto per_sm = [&](int64_t tiles) { return (double)((tiles + sms - 1) / sms); };
+    const int64_t rows_thin = ((int64_t)M + 7) / 8;
+    return rows_thin <= 65535 && 25.0 + 23.0 * per_sm(rows_thin * (((int64_t)N + 31) / 32)) <
+                                     320.0 * per_sm(((int64_t)M + BM - 1) / BM * (((int64_t)N + BN - 1) / BN));
+}
+
 int run_mm(const float* a, const float* b, float* c, int64_t batch, int M, int N, int K, const AnyFmt& gadd, const AnyFmt& gmul_in,
            int rbits_add, int rbits_mul, bool fma_in, int algo, uint64_t seed, void* workspace, size_t workspace_bytes,
            cudaStream_t st, int resume = 0) {
@@ -126,7 +150,9 @@ int run_mm(const float* a, const float* b, float* c, int64_t batch, int M, int N
     // formats whose sums fit a 16-bit register: the same bits from a third to a half of the arithmetic (gemm16_kernel.cuh)
     p.kind16 = (p.stats != nullptr && algo != ALGO_SR && use_packed()) ? kind16_of(fadd, fmul, fma) : -1;
     if (p.kind16 >= 0) {
-        const int rc = small ? launch_mm16_small(algo, p, batch, st) : launch_mm16(algo, p, batch, st);
+        const Tile16 tile = pick_tile16(M, N, batch, algo != ALGO_KAHAN);
+        const int rc = tile == TILE16_THIN ? launch_mm16_thin(algo, p, batch, st)
+                     : tile == TILE16_MID ? launch_mm16_mid(algo, p, batch, st) : launch_mm16(algo, p, batch, st);
         return (rc || !defer) ? rc : launch_mm_exact(algo, fma, p, batch, st);
     }
     if (nosub && p.stats != nullptr) {
@@ -257,7 +283,7 @@ int run_conv_wgrad(const float* gout, const float* x, float* gw, int n_img, int 
         // fewer 128-row tiles than SMs: the 16-row instantiation spreads the same outputs over eight times the CTAs
         const int64_t big_tiles = (((int64_t)p.M + BM - 1) / BM) * (((int64_t)p.N + BN - 1) / BN);
         const bool small = big_tiles < sm_count() && ((int64_t)p.M + kSmallTileRows - 1) / kSmallTileRows <= 65535;
-        const int rc = p.kind16 >= 0 ? (small ? launch_conv16_wgrad_small(algo, p, st) : launch_conv16_wgrad(algo, p, st))
+        const int rc = p.kind16 >= 0 ? (thin_wgrad16(p.M, p.N) ? launch_conv16_wgrad_thin(algo, p, st) : launch_conv16_wgrad(algo, p, st))
                      : small ? launch_conv_wgrad_small_any(algo, fma, p, st) : launch_conv_wgrad_any(algo, fma, p, st);
         if (rc) return rc;
     }

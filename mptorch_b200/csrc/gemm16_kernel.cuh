@@ -166,13 +166,41 @@ __device__ __forceinline__ bool any_small16(uint32_t below, uint32_t min_norm) {
     return (below & 0xFFFFu) < lim || (below >> 16) < lim;
 }
 
-// ---- eight steps -----------------------------------------------------------------------------------------------------
-// Eight steps from slab row kbase for the thread's TM x 4 outputs.  START: the sums start from zero, so the first step
-// is the product itself (an add-format value) and needs no addition.  Returns true when a sum without subnormals has met
-// a value that needs settling: the caller discards the sums and redoes the group on the exact casters.
+// ---- steps -------------------------------------------------------------------------------------------------------------
+// One accumulation step of a pair.  PAIRED: the 32-bit operations as packed fp32x2 instructions (which want the A element
+// twice in a register pair), or as two scalar ones (for threads with few outputs per A element).
+template <bool PAIRED> __device__ __forceinline__ float2 mul2(float a, float2 b) {
+    return PAIRED ? __fmul2_rn(make_float2(a, a), b) : make_float2(mul_rn(a, b.x), mul_rn(a, b.y));
+}
+template <bool PAIRED> __device__ __forceinline__ float2 fma2(float a, float2 b, float2 c) {
+    return PAIRED ? __ffma2_rn(make_float2(a, a), b, c) : make_float2(fma_rn(a, b.x, c.x), fma_rn(a, b.y, c.y));
+}
+// `first`: the sum starts from zero, so it is the product itself (an add-format value) and needs no addition.
+template <int SUM, int PROD, bool NOSUB, bool PAIRED>
+__device__ __forceinline__ uint32_t step16(uint32_t s, float a, float2 b, bool first, const Settle16& ns, uint32_t& below) {
+    if (PROD == PROD16_FUSED) return first ? round16<SUM>(mul2<PAIRED>(a, b)) : round16<SUM>(fma2<PAIRED>(a, b, unpack16<SUM>(s)));
+    const float2 q = mul2<PAIRED>(a, b);
+    if (!NOSUB) {
+        const uint32_t v = prod16<SUM, PROD>(q);
+        return first ? v : sum16<SUM>(s, v);
+    }
+    const float2 keep = settle_keep16(ns, q);
+    const uint32_t r = h2_maxabs(PROD == PROD16_E5M2 ? f2_round_e5m2(q) : PROD == PROD16_E4M3 ? f2_round_e4m3(q) : f2_to_h2(q), ns.min_norm);
+    if (SUM == SUM16_BF16) {
+        const uint32_t v = f2_to_b2(__fmul2_rn(h2_to_f2(r), keep));
+        return first ? v : b2_add(s, v);
+    }
+    const uint32_t k2 = f2_to_h2(keep);
+    s = first ? h2_fma(r, k2, 0u) : settle_sum16<SUM>(h2_fma(r, k2, s));       // + 0: a sum from zero is never -0
+    if (sum_can_settle16(SUM, PROD) && !first) note_small16(below, s);
+    return s;
+}
+
+// Eight steps from slab row kbase for the thread's TM x 4 outputs.  START: the sums start from zero.  Returns true when a
+// sum without subnormals has met a value that needs settling: the caller discards the sums and redoes the group on the
+// exact casters.
 template <int SUM, int PROD, bool START, bool NOSUB>
 __device__ __forceinline__ bool group16(uint32_t (&acc)[TM][2], const float* As, const float* Bs, int kbase, int ty, int tx, const Settle16& ns) {
-    constexpr bool kWatch = NOSUB && sum_can_settle16(SUM, PROD);
     uint32_t below = 0xFFFFFFFFu;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -186,35 +214,12 @@ __device__ __forceinline__ bool group16(uint32_t (&acc)[TM][2], const float* As,
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
                 const float a = j == 0 ? av[i].x : j == 1 ? av[i].y : j == 2 ? av[i].z : av[i].w;
-                const float2 a2 = make_float2(a, a);
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const float2 b2 = c == 0 ? make_float2(bv.x, bv.y) : make_float2(bv.z, bv.w);
-                    uint32_t s = acc[i][c];
-                    if (PROD == PROD16_FUSED) {
-                        s = first ? round16<SUM>(__fmul2_rn(a2, b2)) : round16<SUM>(__ffma2_rn(a2, b2, unpack16<SUM>(s)));
-                    } else if (NOSUB) {
-                        const float2 q = __fmul2_rn(a2, b2);
-                        const float2 keep = settle_keep16(ns, q);
-                        const uint32_t r = h2_maxabs(PROD == PROD16_E5M2 ? f2_round_e5m2(q) : PROD == PROD16_E4M3 ? f2_round_e4m3(q) : f2_to_h2(q), ns.min_norm);
-                        if (SUM == SUM16_BF16) {
-                            const uint32_t v = f2_to_b2(__fmul2_rn(h2_to_f2(r), keep));
-                            s = first ? v : b2_add(s, v);
-                        } else {
-                            const uint32_t k2 = f2_to_h2(keep);
-                            s = first ? h2_fma(r, k2, 0u) : settle_sum16<SUM>(h2_fma(r, k2, s));       // + 0: a sum from zero is never -0
-                        }
-                        if (kWatch && !first) note_small16(below, s);
-                    } else {
-                        const uint32_t v = prod16<SUM, PROD>(__fmul2_rn(a2, b2));
-                        s = first ? v : sum16<SUM>(s, v);
-                    }
-                    acc[i][c] = s;
-                }
+                acc[i][0] = step16<SUM, PROD, NOSUB, true>(acc[i][0], a, make_float2(bv.x, bv.y), first, ns, below);
+                acc[i][1] = step16<SUM, PROD, NOSUB, true>(acc[i][1], a, make_float2(bv.z, bv.w), first, ns, below);
             }
         }
     }
-    return kWatch && any_small16(below, ns.min_norm);
+    return NOSUB && sum_can_settle16(SUM, PROD) && any_small16(below, ns.min_norm);
 }
 
 // Eight compensated steps (kahan_fast2 in gemm_kernel.cuh, on pairs): acc = running sums, nc = negated compensation terms.
@@ -288,7 +293,7 @@ __device__ __forceinline__ void negate_all(float (&f)[TM][TN]) {      // zeros b
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------------------
-// Tiling, staging and epilogue are mm_kernel's: 128 x 64 outputs per CTA (16 x 64 in gemm16_small.cu), 256 threads, 8 x 4
+// Tiling, staging and epilogue are mm_kernel's: 128 x 64 outputs per CTA (64 x 64 in gemm16_mid.cu), 256 threads, 8 x 4
 // outputs per thread as 16 pairs, K slabs of 32 through three cp.async stages.
 template <int ALGO, int SUM, int PROD, bool NOSUB, int CONV, int MINB, int TILE_ROWS = BM>
 __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_constant__ MmParams p) {
@@ -475,26 +480,23 @@ int launch_one16(const MmParams& p, int64_t batch, cudaStream_t st) {
     kern<<<grid, THREADS, smem, st>>>(p);
     return check_launch("float_mm");
 }
-template <int ALGO, int CONV, int MINB, int TILE_ROWS = BM>
-int launch_any16(const MmParams& p, int64_t batch, cudaStream_t st) {
-#define MPT_KIND16(S, P) case kind16(S, P): return launch_one16<ALGO, S, P, CONV, MINB, TILE_ROWS>(p, batch, st);
-    switch (p.kind16) {
-        MPT_KIND16(SUM16_F16, PROD16_E5M2)
-        MPT_KIND16(SUM16_F16, PROD16_E4M3)
-        MPT_KIND16(SUM16_F16, PROD16_F16)
-        MPT_KIND16(SUM16_F16, PROD16_FUSED)
-        MPT_KIND16(SUM16_BF16, PROD16_E5M2)
-        MPT_KIND16(SUM16_BF16, PROD16_E4M3)
-        MPT_KIND16(SUM16_BF16, PROD16_BF16)
-        MPT_KIND16(SUM16_BF16, PROD16_FUSED)
-        MPT_KIND16(SUM16_E5M2, PROD16_E5M2)
-        MPT_KIND16(SUM16_E5M2, PROD16_FUSED)
-        MPT_KIND16(SUM16_E4M3, PROD16_E4M3)
-        MPT_KIND16(SUM16_E4M3, PROD16_FUSED)
-    }
-#undef MPT_KIND16
+// One case per format pair of kind16_of.
+#define MPT_KINDS16(CASE)                                                                                                 \
+    CASE(SUM16_F16, PROD16_E5M2) CASE(SUM16_F16, PROD16_E4M3) CASE(SUM16_F16, PROD16_F16) CASE(SUM16_F16, PROD16_FUSED)      \
+    CASE(SUM16_BF16, PROD16_E5M2) CASE(SUM16_BF16, PROD16_E4M3) CASE(SUM16_BF16, PROD16_BF16) CASE(SUM16_BF16, PROD16_FUSED) \
+    CASE(SUM16_E5M2, PROD16_E5M2) CASE(SUM16_E5M2, PROD16_FUSED) CASE(SUM16_E4M3, PROD16_E4M3) CASE(SUM16_E4M3, PROD16_FUSED)
+inline int no_kind16(const MmParams& p) {
     set_error("float_mm: no 16-bit kernel for kind %d", p.kind16);
     return MPT_ERR_INVALID_ARGUMENT;
+}
+template <int ALGO, int CONV, int MINB, int TILE_ROWS = BM>
+int launch_any16(const MmParams& p, int64_t batch, cudaStream_t st) {
+    switch (p.kind16) {
+#define MPT_CASE16(S, P) case kind16(S, P): return launch_one16<ALGO, S, P, CONV, MINB, TILE_ROWS>(p, batch, st);
+        MPT_KINDS16(MPT_CASE16)
+#undef MPT_CASE16
+    }
+    return no_kind16(p);
 }
 
 }  // namespace mpt

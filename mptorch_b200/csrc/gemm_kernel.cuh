@@ -1036,10 +1036,11 @@ int launch_mm_exact(int algo, bool fma, const MmParams& p, int64_t batch, cudaSt
 int launch_mm_nosub(int algo, bool fma, const MmParams& p, int64_t batch, bool vec, cudaStream_t st);  // ALGO_SEQ / ALGO_TILE8
 // The same products on 16-bit running sums (gemm16_kernel.cuh), for p.kind16 >= 0.
 int launch_mm16(int algo, const MmParams& p, int64_t batch, cudaStream_t st);                            // all but ALGO_SR
-int launch_mm16_small(int algo, const MmParams& p, int64_t batch, cudaStream_t st);                      // ALGO_SEQ / ALGO_TILE8
+int launch_mm16_mid(int algo, const MmParams& p, int64_t batch, cudaStream_t st);
+int launch_mm16_thin(int algo, const MmParams& p, int64_t batch, cudaStream_t st);                       // ALGO_SEQ / ALGO_TILE8
 int launch_conv16(int algo, const MmParams& p, cudaStream_t st);
 int launch_conv16_wgrad(int algo, const MmParams& p, cudaStream_t st);
-int launch_conv16_wgrad_small(int algo, const MmParams& p, cudaStream_t st);
+int launch_conv16_wgrad_thin(int algo, const MmParams& p, cudaStream_t st);
 constexpr int kSmallTileRows = 16;      // tile height of the instantiation behind launch_conv_wgrad_small_any
 
 }  // namespace mpt
