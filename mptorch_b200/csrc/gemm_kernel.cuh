@@ -34,6 +34,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "async_copy.cuh"
 #include "cast.cuh"
 #include "common.cuh"
 
@@ -197,18 +198,6 @@ static __global__ void __launch_bounds__(256) stats_kernel(const float* __restri
         atomicMin(mn, lmin);
     }
 }
-
-__device__ __forceinline__ void cp_async16(float* dst, const float* src, int src_bytes) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async4(float* dst, const float* src, int src_bytes) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // Stage one K slab: As[m][k] (row stride AS_LD) and Bs[k][n].  Elements outside the matrices are
 // zero filled (cp.async with a source size of 0), which is also how K is zero padded.

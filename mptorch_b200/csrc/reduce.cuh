@@ -516,4 +516,11 @@ void launch_layernorm_fwd_rows(const float* in, const float* weight, const float
 void launch_layernorm_bwd_rows(const float* in, const float* grad_out, const float* weight, const float* mean, const float* rstd,
                                float* grad_in, const RowGeom& g, const LnFmt& f, int mode, const RowLimits& lim, void* stream);
 
+// Column chains on 16-bit sums and column sums over few rows (colsum16.cu); mode as in colsum_kernel.
+bool chain16_ok(const Caster& acc);
+int launch_chain16(int mode, const float* in, const float* gout, const float* mean, const float* rstd, float* out0, float* out1,
+                   const RowGeom& g, const Caster& facc, const Caster& fmul, cudaStream_t st, const char* who);
+bool wide_colsum_ok(const RowGeom& g);
+int launch_wide_colsum(const float* in, float* out, const RowGeom& g, const SeqAdder& seq, cudaStream_t st, const char* who);
+
 }  // namespace mpt
