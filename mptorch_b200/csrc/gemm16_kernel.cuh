@@ -252,6 +252,12 @@ __device__ __forceinline__ void kahan_group16(uint32_t (&acc)[TM][2], uint32_t (
     }
 }
 
+// A magnitude limit as a 16-bit pattern of the sums' type, rounded down; 0 (which no sum is below) where there is none.
+template <int SUM>
+__device__ __forceinline__ uint32_t limit16(float limit) {
+    const float l = fmaxf(limit, 0.0f);
+    return SUM == SUM16_BF16 ? (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rd(l)) : (uint32_t)__half_as_ushort(__float2half_rd(l));
+}
 // Largest |x| of the thread's pairs is below `lim` (a 16-bit pattern of the sums' type, itself not above the limit)?
 template <int SUM>
 __device__ __forceinline__ bool all_below16(const uint32_t (&v)[TM][2], uint32_t lim) {
@@ -325,8 +331,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
     const int ksteps = plan.ok && (ALGO == ALGO_SEQ || (ALGO == ALGO_TILE8 && !kFlush)) ? (p.K + 7) / 8 * 8
                      : (ALGO == ALGO_SEQ || (p.resume & MM_MORE)) ? p.K : p.K + 8 - p.K % 8;
     const int ntiles = (ksteps + BK - 1) / BK;
-    const uint32_t lim = SUM == SUM16_BF16 ? (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rd(plan.acc_limit))
-                                           : (uint32_t)__half_as_ushort(__float2half_rd(plan.acc_limit));
+    const uint32_t lim = limit16<SUM>(plan.acc_limit), slab_lim = limit16<SUM>(plan.slab_limit);
     const Settle16 ns = Settle16::make(p.fmul);
 
     if (CONV == CONV_FWD) {
@@ -354,8 +359,21 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
             }
     }
 
+    // a tile inside the matrix needs no bounds: one address and a constant step per thread
+    const bool inside = CONV == CONV_NONE && p.vec && m0 + BM <= p.M && n0 + BN <= p.N;
+    const float* a_src = A + (int64_t)(m0 + (tid >> 3)) * p.K + ((tid & 7) << 2);
+    const float* b_src = B + (int64_t)(tid >> 4) * p.N + n0 + ((tid & 15) << 2);
     auto stage = [&](int s, int k0) {
-        if (CONV == CONV_NONE && p.vec) load_tiles<true, CONV_NONE>(p, A, B, As + s * SMEM_A, Bs + s * SMEM_B, m0, n0, k0, tid, crow);
+        if (inside && BM >= 32 && k0 + BK <= p.K) {
+            const float* a = a_src + k0;
+            const float* b = b_src + (int64_t)k0 * p.N;
+            float* as = As + s * SMEM_A + (tid >> 3) * AS_LD + ((tid & 7) << 2);
+            float* bs = Bs + s * SMEM_B + (tid >> 4) * BN + ((tid & 15) << 2);
+#pragma unroll
+            for (int u = 0; u < BM / 32; ++u) cp_async16(as + 32 * u * AS_LD, a + (int64_t)(32 * u) * p.K, 16);
+#pragma unroll
+            for (int u = 0; u < BK / 16; ++u) cp_async16(bs + 16 * u * BN, b + (int64_t)(16 * u) * p.N, 16);
+        } else if (CONV == CONV_NONE && p.vec) load_tiles<true, CONV_NONE>(p, A, B, As + s * SMEM_A, Bs + s * SMEM_B, m0, n0, k0, tid, crow);
         else load_tiles<false, CONV>(p, A, B, As + s * SMEM_A, Bs + s * SMEM_B, m0, n0, k0, tid, crow);
     };
 #pragma unroll
@@ -375,6 +393,8 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
         const float* as = As + (t % STAGES) * SMEM_A;
         const float* bs = Bs + (t % STAGES) * SMEM_B;
         const int nk_tile = min(ksteps - t * BK, BK);
+        // one look at the sums for the slab's four groups; where it does not suffice every group looks for itself
+        const bool slab_ok = ALGO != ALGO_KAHAN && !(wide_start && t == 0) && all_below16<SUM>(ALGO == ALGO_TILE8 ? aux : acc, slab_lim);
 #pragma unroll 1
         for (int g = 0; g * 8 < nk_tile; ++g) {
             const int nk = min(nk_tile - g * 8, 8);
@@ -393,7 +413,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
                 }
                 // fold the group into the outer sum
                 bool folded = false;
-                if (plan.ok && !wide && all_below16<SUM>(aux, lim)) {
+                if (plan.ok && !wide && (slab_ok || all_below16<SUM>(aux, lim))) {
                     uint32_t below = 0xFFFFFFFFu, out[TM][2];
 #pragma unroll
                     for (int i = 0; i < TM; ++i)
@@ -421,7 +441,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
             } else if (ALGO == ALGO_SEQ) {
                 bool redo = true;
                 const int kleft = p.K - t * BK - g * 8;
-                if (plan.ok && !wide && all_below16<SUM>(acc, lim) && !(kFlush && kleft < 8 && any_minus_zero16(acc))) {
+                if (plan.ok && !wide && (slab_ok || all_below16<SUM>(acc, lim)) && !(kFlush && kleft < 8 && any_minus_zero16(acc))) {
                     uint32_t saved[TM][2];
                     if (kFlush) {
 #pragma unroll

@@ -634,7 +634,8 @@ __device__ __forceinline__ float absmax_of(const float (&v)[TM][TN]) {
 //               no fp32-denormal intermediates where the reference treats those specially)
 //   acc_limit : an accumulator with |acc| below this stays on the fast path for 8 more steps
 //               (ALGO_SEQ), or an outer sum below this takes the fast fold (ALGO_TILE8)
-struct FastPlan { bool ok; float acc_limit; };
+//   slab_limit: the same for four groups (32 steps); not positive where that cannot be promised
+struct FastPlan { bool ok; float acc_limit, slab_limit; };
 
 // Formats without subnormals qualify when the launch is of the NOSUB instantiation (the host decides; the kernel's
 // roundings then settle what lands below the smallest normal value the way the reference does).
@@ -642,7 +643,7 @@ __host__ __device__ inline bool mm_fast_format_nosub(const FpFmt& f) { return !f
 
 template <int ALGO, bool FMA>
 __device__ __forceinline__ FastPlan make_plan(const MmParams& p, int64_t batch) {
-    FastPlan plan{false, 0.0f};
+    FastPlan plan{false, 0.0f, 0.0f};
     if (p.stats == nullptr) return plan;
     const MmStats s = p.stats[batch];
     if (s.max_a >= 0x7F800000u || s.max_b >= 0x7F800000u) return plan;
@@ -694,11 +695,13 @@ __device__ __forceinline__ FastPlan make_plan(const MmParams& p, int64_t batch) 
         if (!(step8 <= ldexpf(1.0f, lim_add))) return plan;
         plan.ok = true;
         plan.acc_limit = ldexpf(1.0f, lim_add);
+        plan.slab_limit = plan.acc_limit / p.growth8 - 3.0f * step8;      // three folds before the last one
     } else {
         const float lim = top / p.growth8 - ldexpf(8.0f, pe);
         if (!(lim > 0.0f)) return plan;
         plan.ok = true;
         plan.acc_limit = lim;
+        plan.slab_limit = top / (p.growth8 * p.growth8 * p.growth8 * p.growth8) - ldexpf(32.0f, pe);
     }
     return plan;
 }
