@@ -120,17 +120,7 @@ int run_mm(const float* a, const float* b, float* c, int64_t batch, int M, int N
                                 (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0 && K > 0;
     if (fast_candidate) {
         MmStats* s = static_cast<MmStats*>(workspace);
-        stats_init_kernel<<<(unsigned)((batch + 255) / 256), 256, 0, st>>>(s, batch);
-        const int64_t na = (int64_t)M * K, nb = (int64_t)K * N;
-        const int sms = sm_count();
-        auto grid = [&](int64_t n) {
-            int64_t g = (n + 255) / 256;
-            const int64_t cap = ((int64_t)sms * 8 + batch - 1) / batch;
-            return dim3((unsigned)(g > cap ? cap : (g < 1 ? 1 : g)), (unsigned)batch);
-        };
-        stats_kernel<<<grid(na), 256, 0, st>>>(a, na, s, 0);
-        stats_kernel<<<grid(nb), 256, 0, st>>>(b, nb, s, 1);
-        int rc = check_launch("float_mm statistics");
+        const int rc = launch_mm_stats(a, (int64_t)M * K, b, (int64_t)K * N, batch, s, st);
         if (rc) return rc;
         p.stats = s;
     }
@@ -209,13 +199,7 @@ int run_conv(const float* x, const float* wt, float* y, int n_img, int c_in, int
     if (fast_candidate) {
         // one record for all groups: the maxima over the whole input and the whole weight bound every group's products
         MmStats* s = static_cast<MmStats*>(workspace);
-        stats_init_kernel<<<1, 256, 0, st>>>(s, 1);
-        const int64_t nx = (int64_t)n_img * c_in * H * W, nw = (int64_t)c_out * K64;
-        const int sms = sm_count();
-        auto grid = [&](int64_t n) { int64_t g = (n + 255) / 256; const int64_t cap = (int64_t)sms * 8; return dim3((unsigned)(g > cap ? cap : (g < 1 ? 1 : g)), 1); };
-        stats_kernel<<<grid(nx), 256, 0, st>>>(x, nx, s, 0);
-        stats_kernel<<<grid(nw), 256, 0, st>>>(wt, nw, s, 1);
-        int rc = check_launch("float_conv2d statistics");
+        const int rc = launch_mm_stats(x, (int64_t)n_img * c_in * H * W, wt, (int64_t)c_out * K64, 1, s, st);
         if (rc) return rc;
         p.stats = s;
     }
@@ -266,13 +250,7 @@ int run_conv_wgrad(const float* gout, const float* x, float* gw, int n_img, int 
     p.kind16 = (fast_candidate && use_packed()) ? kind16_of(fadd, p.fmul, fma) : -1;
     if (fast_candidate) {
         MmStats* s = static_cast<MmStats*>(workspace);
-        stats_init_kernel<<<1, 256, 0, st>>>(s, 1);
-        const int64_t ng = (int64_t)n_img * c_out * L, nx = (int64_t)n_img * c_in * H * W;
-        const int sms = sm_count();
-        auto grid = [&](int64_t n) { int64_t g = (n + 255) / 256; const int64_t cap = (int64_t)sms * 8; return dim3((unsigned)(g > cap ? cap : (g < 1 ? 1 : g)), 1); };
-        stats_kernel<<<grid(ng), 256, 0, st>>>(gout, ng, s, 0);
-        stats_kernel<<<grid(nx), 256, 0, st>>>(x, nx, s, 1);
-        int rc = check_launch("float_conv2d_wgrad statistics");
+        const int rc = launch_mm_stats(gout, (int64_t)n_img * c_out * L, x, (int64_t)n_img * c_in * H * W, 1, s, st);
         if (rc) return rc;
         p.stats = s;
     }

@@ -60,7 +60,7 @@ constexpr size_t SMEM_BYTES = (size_t)STAGES * (SMEM_A + SMEM_B) * sizeof(float)
 
 enum Algo : int { ALGO_SEQ = 0, ALGO_TILE8 = 1, ALGO_KAHAN = 2, ALGO_SR = 3 };
 
-// Magnitude statistics of the operands, produced by stats_kernel into the workspace.
+// Magnitude statistics of the operands, produced by gemm_stats.cu into the workspace.
 struct MmStats {
     uint32_t max_a, max_b;       // largest |x| bit pattern (NaN and inf compare above every finite)
     uint32_t minnz_a, minnz_b;   // smallest nonzero |x| bit pattern, 0xFFFFFFFF if all zero
@@ -163,41 +163,8 @@ __device__ __forceinline__ float sr_mul(const MmParams& p, float x, uint32_t r) 
     return p.sr_ok ? p.smul(x, r) : cast_fp_stochastic(x, r, p.rbits_mul, p.fmul);
 }
 
-static __global__ void stats_init_kernel(MmStats* s, int64_t batch) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < batch) { s[i].max_a = 0u; s[i].max_b = 0u; s[i].minnz_a = 0xFFFFFFFFu; s[i].minnz_b = 0xFFFFFFFFu; }
-}
-
-// blockIdx.y walks the batch; `which` selects the A (0) or B (1) fields of that entry's record.
-static __global__ void __launch_bounds__(256) stats_kernel(const float* __restrict__ base, int64_t n, MmStats* stats, int which) {
-    const float* x = base + (int64_t)blockIdx.y * n;
-    uint32_t* mx = which ? &stats[blockIdx.y].max_b : &stats[blockIdx.y].max_a;
-    uint32_t* mn = which ? &stats[blockIdx.y].minnz_b : &stats[blockIdx.y].minnz_a;
-    uint32_t lmax = 0u, lmin = 0xFFFFFFFFu;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    auto take = [&](float v) {
-        const uint32_t a = __float_as_uint(v) & 0x7FFFFFFFu;
-        lmax = max(lmax, a);
-        lmin = min(lmin, a - 1u);                      // zero wraps to the largest value and so never wins
-    };
-    // 16-byte loads, four in flight per thread, where this entry starts on a 16-byte boundary
-    const int64_t n4 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 ? n / 4 : 0;
-    const float4* x4 = reinterpret_cast<const float4*>(x);
-#pragma unroll 4
-    for (int64_t i = tid; i < n4; i += stride) {
-        const float4 v = x4[i];
-        take(v.x); take(v.y); take(v.z); take(v.w);
-    }
-    for (int64_t i = 4 * n4 + tid; i < n; i += stride) take(x[i]);
-    lmin = lmin == 0xFFFFFFFFu ? lmin : lmin + 1u;     // back from (pattern - 1); all zero stays 0xFFFFFFFF
-    lmax = __reduce_max_sync(0xFFFFFFFFu, lmax);
-    lmin = __reduce_min_sync(0xFFFFFFFFu, lmin);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(mx, lmax);
-        atomicMin(mn, lmin);
-    }
-}
+// Fills one record per batch entry: na elements of A and nb of B each (gemm_stats.cu).
+int launch_mm_stats(const float* a, int64_t na, const float* b, int64_t nb, int64_t batch, MmStats* stats, cudaStream_t st);
 
 // Stage one K slab: As[m][k] (row stride AS_LD) and Bs[k][n].  Elements outside the matrices are
 // zero filled (cp.async with a source size of 0), which is also how K is zero padded.
