@@ -79,6 +79,14 @@ MPT_API int mpt_copy_columns_async(void *dst, size_t dst_pitch, const void *src,
  * batch and rows / 64 are limited to 65535. */
 MPT_API int mpt_transpose_last2(const float *in, float *out, int64_t batch, int64_t rows, int64_t cols, void *stream);
 
+/* No counterpart in the reference (its conv.py:591-640 leaves the folding of the unfolded input's gradient to autograd).
+ * The input gradient of a convolution from the gradient of its unfolded input: cols is [n_img, OH * OW, channels * KH * KW],
+ * out one [channels, H, W] image per n_img, out_image_stride floats apart; every pixel is the fp32 sum, from zero, of its
+ * copies' entries in ascending output position, which is what F.fold computes.  One pixel's output positions have to fit
+ * 96 KB of shared memory: (floor((KH - 1) * dil_h / stride_h) + 1) * (the same for the width) * (KH * KW + 1) <= 24576. */
+MPT_API int mpt_fold(const float *cols, float *out, int n_img, int channels, int H, int W, int KH, int KW, int stride_h,
+                     int stride_w, int pad_h, int pad_w, int dil_h, int dil_w, int64_t out_image_stride, void *stream);
+
 /* ---- elementwise quantizers ------------------------------------------------------------- */
 
 /* replaces float_quantize_nearest (pybind_cuda.cpp:44 -> quant.cu:143 -> fp_kernel.cu:164) */

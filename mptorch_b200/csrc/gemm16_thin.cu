@@ -6,11 +6,12 @@
 // the weight gradient of a 3 x 3 layer of 64 channels (64 x 576 outputs) becomes 144 CTAs for 148 SMs, one warp per
 // scheduler.  In the CUDA order four groups of eight steps run at once (their inner sums start from zero), so that the
 // conversions' latencies overlap.  K slabs of 64 through three cp.async stages.  Against 16 x 64 tiles of mm16_kernel
-// (1 x 4 outputs per thread): 256 x 256 x 4096 170 -> 114 us, that gradient 10.0 -> 4.9 ms, 64 x 64 x 1024 36 -> 30 us.
+// (1 x 4 outputs per thread): 256 x 256 x 4096 170 -> 114 us, that gradient 10.0 -> 4.0 ms (4.9 while the computing warps staged), 64 x 64 x 1024 36 -> 30 us.
 //
 // The weight gradient of a convolution gathers B from the input (CONV_WGRAD): a lane owns two output positions of the slab,
 // walks them forward slab by slab without divisions, and copies them for eight of the tile's columns (channel, kernel
-// row, kernel column), so that a warp's 32 copies are neighbouring pixels.
+// row, kernel column), so that a warp's 32 copies are neighbouring pixels.  Its address arithmetic is as long as the sums
+// themselves, and with one warp per scheduler nothing covers it, so four more warps of the CTA do the staging.
 #include "gemm16_kernel.cuh"
 
 namespace mpt {
@@ -19,6 +20,7 @@ namespace {
 constexpr int TBM = 8, TBN = 32, TBK = 64, TTHREADS = 128, TSTAGES = 3;
 constexpr int kRun = 4;         // groups of eight steps in flight per thread (CUDA order)
 constexpr int TA_LD = TBK + 4;
+__host__ __device__ constexpr int stagers(int conv) { return conv == CONV_WGRAD ? TTHREADS : 0; }      // threads that only stage
 __host__ __device__ constexpr int tb_ld(int conv) { return conv == CONV_WGRAD ? TBN + 2 : TBN + 4; }   // 4-byte column writes / 16-byte rows
 
 // `n` steps of a pair on the exact casters: a = the thread's row of the A slab, b = its column pair of the B slab.
@@ -76,7 +78,7 @@ struct Position {
 struct Column { int64_t off; int dih, diw; };       // input offset of (channel, kernel row, kernel column); rows past N: dih out of every image
 
 template <int ALGO, int SUM, int PROD, bool NOSUB, int CONV>
-__global__ void __launch_bounds__(TTHREADS, 6) mm16_thin_kernel(const __grid_constant__ MmParams p) {
+__global__ void __launch_bounds__(TTHREADS + stagers(CONV), CONV == CONV_WGRAD ? 3 : 6) mm16_thin_kernel(const __grid_constant__ MmParams p) {
     constexpr bool FMA = PROD == PROD16_FUSED;
     constexpr bool kFlush = NOSUB && sum_can_settle16(SUM, PROD);
     constexpr int LDB = tb_ld(CONV);
@@ -84,7 +86,8 @@ __global__ void __launch_bounds__(TTHREADS, 6) mm16_thin_kernel(const __grid_con
     __shared__ __align__(16) float Bs[TSTAGES][TBK * LDB];
     __shared__ Column cols[CONV == CONV_WGRAD ? TBN : 1];
 
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const bool computes = threadIdx.x < TTHREADS, stages = stagers(CONV) == 0 || !computes;
+    const int tid = threadIdx.x & (TTHREADS - 1), ty = tid >> 4, tx = tid & 15;
     const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
     const int64_t batch = blockIdx.z;
     const float* A = p.a + batch * p.stride_a;
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(TTHREADS, 6) mm16_thin_kernel(const __grid_con
     const int L = CONV == CONV_WGRAD ? p.cv.OH * p.cv.OW : 1;
     Position pos[2];
     if (CONV == CONV_WGRAD) {
-        if (tid < TBN) {
+        if (computes && tid < TBN) {
             const int gj = n0 + tid, khkw = p.cv.KH * p.cv.KW;
             const int ch = gj / khkw, rem = gj - ch * khkw, kh = rem / p.cv.KW, kw = rem - kh * p.cv.KW;
             Column c;
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(TTHREADS, 6) mm16_thin_kernel(const __grid_con
 
 #pragma unroll
     for (int s = 0; s < TSTAGES - 1; ++s) {
-        if (s < ntiles) stage(s, s * TBK);
+        if (stages && s < ntiles) stage(s, s * TBK);
         cp_async_commit();
     }
     int slot = 0;
@@ -204,11 +207,14 @@ __global__ void __launch_bounds__(TTHREADS, 6) mm16_thin_kernel(const __grid_con
         __syncthreads();
         {
             const int nt = t + TSTAGES - 1;
-            if (nt < ntiles) stage(slot == 0 ? TSTAGES - 1 : slot - 1, nt * TBK);
+            if (stages && nt < ntiles) stage(slot == 0 ? TSTAGES - 1 : slot - 1, nt * TBK);
             cp_async_commit();
         }
-        const float* arow = As[slot] + ty * TA_LD;
-        const float* bcol = Bs[slot] + 2 * tx;
+        const int now = slot;
+        slot = slot == TSTAGES - 1 ? 0 : slot + 1;
+        if (!computes) continue;
+        const float* arow = As[now] + ty * TA_LD;
+        const float* bcol = Bs[now] + 2 * tx;
         const int nk_tile = min(ksteps - t * TBK, TBK);
         int k0 = 0;
         // Several groups at once: the inner sums of the CUDA order start from zero, so four groups are four independent chains
@@ -264,13 +270,12 @@ __global__ void __launch_bounds__(TTHREADS, 6) mm16_thin_kernel(const __grid_con
                 if (redo) acc = pack16<SUM>(thin_exact_steps<FMA>(wide ? c_in : unpack16<SUM>(saved), ak, bk, LDB, min(min(nk_tile - k0, 8), kleft), &p));
             }
         }
-        slot = slot == TSTAGES - 1 ? 0 : slot + 1;
     }
     cp_async_wait<0>();
 
     float2 r = unpack16<SUM>(ALGO == ALGO_TILE8 ? aux : acc);
     if (ALGO == ALGO_SEQ && FMA && SUM != SUM16_BF16) r = make_float2(add_rn(r.x, 0.0f), add_rn(r.y, 0.0f));      // conversions round to -0 as well
-    if (gm >= p.M) return;
+    if (!computes || gm >= p.M) return;
     float* dst = C + (int64_t)gm * p.N + gn;
     if (gn < p.N) dst[0] = r.x;
     if (gn + 1 < p.N) dst[1] = r.y;
@@ -281,8 +286,8 @@ int launch_thin_one(const MmParams& p, int64_t batch, cudaStream_t st) {
     constexpr bool kNosub = PROD != PROD16_FUSED && settles16(SUM, PROD);
     const dim3 grid((unsigned)((p.N + (int64_t)TBN - 1) / TBN), (unsigned)((p.M + (int64_t)TBM - 1) / TBM), (unsigned)batch);
     if (grid.y > 65535u) { set_error("float_mm: M=%d has more than 65535 row tiles of %d", p.M, TBM); return MPT_ERR_INVALID_ARGUMENT; }
-    if (kNosub && p.nosub) mm16_thin_kernel<ALGO, SUM, PROD, kNosub, CONV><<<grid, TTHREADS, 0, st>>>(p);
-    else mm16_thin_kernel<ALGO, SUM, PROD, false, CONV><<<grid, TTHREADS, 0, st>>>(p);
+    if (kNosub && p.nosub) mm16_thin_kernel<ALGO, SUM, PROD, kNosub, CONV><<<grid, TTHREADS + stagers(CONV), 0, st>>>(p);
+    else mm16_thin_kernel<ALGO, SUM, PROD, false, CONV><<<grid, TTHREADS + stagers(CONV), 0, st>>>(p);
     return check_launch("float_mm");
 }
 template <int ALGO, int CONV>

@@ -10,7 +10,7 @@ import torch
 
 from ..number import FloatingPoint, FloatType
 from .quant_format import QAffineFormats, QLayerNormFormats, QSoftmaxFormats, id_quant, make_quant_function
-from .quant_function import (mp_bmm, mp_layernorm_backward, mp_layernorm_forward, mp_mm, mp_softmax_backward,
+from .quant_function import (_f32c, mp_bmm, mp_layernorm_backward, mp_layernorm_forward, mp_mm, mp_softmax_backward,
                              mp_softmax_forward, qsum_rows)
 
 __all__ = ["qlinear", "qconv2d", "qmm", "qmatmul", "qsoftmax", "qlayernorm", "qsum", "compute_bias", "scale", "unscale"]
@@ -316,6 +316,8 @@ class qconv2d_kernel(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output):
+        from .. import backend as _be
+
         qinput, qweight, qbias = ctx.saved_tensors
         f = ctx.formats
         stride, padding, dilation, groups = ctx.geom
@@ -323,14 +325,12 @@ class qconv2d_kernel(torch.autograd.Function):
         c_out, cg, kh, kw = qweight.shape
         og = c_out // groups
         grad_scale = 0                # the implicit path is taken only without tensor scaling (implicit_conv_eligible)
-        gin, gws, gbs = [], [], []
+        grad_input, gws, gbs = None, [], []
         implicit_w = ctx.needs_input_grad[1] and implicit_wgrad_eligible(f)
         # the implicit weight gradient runs beside the per-group input gradients (its quantizer is deterministic, so
         # the order of the calls does not matter to any random stream)
         second = _second_gradient(grad_output, bool(implicit_w and ctx.needs_input_grad[0]))
         if implicit_w:
-            from .. import backend as _be
-
             with second:
                 qgo_all = f.grad_quant(grad_output).contiguous().float()     # elementwise: the values the per-group path sees
                 gw_all = torch.empty(c_out, cg * kh * kw, device=grad_output.device)
@@ -340,14 +340,19 @@ class qconv2d_kernel(torch.autograd.Function):
                 gws.append(f.grad_quant(gw_all).view(c_out, cg, kh, kw))
         for g in range(groups):
             go = grad_output[:, g * og:(g + 1) * og]
-            go2 = go.reshape(n, og, -1).transpose(1, 2).reshape(-1, og)              # [N * L, og], as qlinear sees it
+            go2 = go.reshape(n, og, -1).transpose(1, 2)
+            go2 = (_f32c(go2) if go2.dtype == torch.float32 else go2).reshape(-1, og)  # [N * L, og], as qlinear sees it
             qgo = f.grad_quant(go2)
             w2 = qweight[g * og:(g + 1) * og].reshape(og, -1)
             if ctx.needs_input_grad[0]:
                 gc = torch.matmul(qgo, w2) if f.bwd_use_default_prec else mp_bmm(qgo, w2, formats=f, use_forward=False)
-                gc = f.grad_quant(gc)
-                gc = gc.view(n, -1, gc.shape[-1]).transpose(1, 2)                    # [N, K, L]
-                gin.append(torch.nn.functional.fold(gc, (h, w), (kh, kw), dilation=dilation, padding=padding, stride=stride))
+                gc = f.grad_quant(gc)                                                # [N * L, K]
+                if grad_input is None:
+                    grad_input = torch.empty(n, c, h, w, device=gc.device, dtype=gc.dtype)
+                if not _be.fold_into(gc, grad_input, g * cg, cg, (kh, kw), stride, padding, dilation):
+                    gc = gc.view(n, -1, gc.shape[-1]).transpose(1, 2)                # [N, K, L]
+                    grad_input[:, g * cg:(g + 1) * cg] = torch.nn.functional.fold(gc, (h, w), (kh, kw), dilation=dilation,
+                                                                                  padding=padding, stride=stride)
             if ctx.needs_input_grad[1] and not implicit_w:
                 cols = _conv_cols(qinput[:, g * cg:(g + 1) * cg], (kh, kw), dilation, padding, stride)
                 gw = (torch.matmul(qgo.transpose(-2, -1), cols) if f.bwd_use_default_prec
@@ -364,7 +369,6 @@ class qconv2d_kernel(torch.autograd.Function):
                             gb = qsum(qgo, dim=(0,), quant=make_quant_function(f.bwd_add, f.bwd_rnd, f.rbits_add))
                 gbs.append(f.grad_quant(gb.reshape(-1)))
         second.join(*gws)
-        grad_input = torch.cat(gin, dim=1) if gin else None
         grad_weight = torch.cat(gws, dim=0) if gws else None
         grad_bias = torch.cat(gbs, dim=0) if gbs else None
         return grad_input, grad_weight, grad_bias, None, None, None, None, None
