@@ -35,7 +35,7 @@ FMT = dict(man_add=2, exp_add=5, man_mul=2, exp_mul=5, subnormals=True, saturate
 # and the git blob hashes of the kernel sources they were taken at; when the sources have changed since, the bench line
 # says so ("constants_stale") instead of silently reporting an old roofline.
 COUNTERS_PATH = os.path.join(ROOT, "profiles", "mm_kernel_counters.json")
-KERNEL_SOURCES = ("mptorch_b200/csrc/gemm_kernel.cuh", "mptorch_b200/csrc/cast.cuh")
+KERNEL_SOURCES = ("mptorch_b200/csrc/gemm16_kernel.cuh", "mptorch_b200/csrc/gemm_kernel.cuh", "mptorch_b200/csrc/cast.cuh")
 
 
 def git_blob_hash(path: str) -> str:
@@ -55,7 +55,7 @@ def load_counters() -> dict:
 def record_counters(per_mac_csv: str, per_mac_size: int, traffic_csv: str | None, note: str) -> dict:
     """Rebuild profiles/mm_kernel_counters.json from ncu `--csv` logs of the GEMM kernel: `per_mac_csv` holds
     smsp__inst_executed.sum, sm__inst_executed_pipe_alu.sum, sm__inst_executed_pipe_fma.sum (and anything else asked for) of
-    one mm_kernel launch at M = N = K = `per_mac_size`; `traffic_csv` dram__bytes_read.sum / dram__bytes_write.sum of one
+    one mm16_kernel launch at M = N = K = `per_mac_size`; `traffic_csv` dram__bytes_read.sum / dram__bytes_write.sum of one
     launch at 8192^3.  The hashes of the kernel sources as they are now are stored beside the numbers."""
     import csv
 
@@ -65,7 +65,7 @@ def record_counters(per_mac_csv: str, per_mac_size: int, traffic_csv: str | None
         head = rows[0]
         ik, im, iv, iu = head.index("Kernel Name"), head.index("Metric Name"), head.index("Metric Value"), head.index("Metric Unit")
         for r in rows[1:]:
-            if "mm_kernel" in r[ik] and r[im] not in out:
+            if "mm16_kernel" in r[ik] and r[im] not in out:
                 v = float(r[iv].replace(",", ""))
                 unit = r[iu].lower()
                 v *= {"kbyte": 1e3, "mbyte": 1e6, "gbyte": 1e9}.get(unit, 1.0)
@@ -84,7 +84,7 @@ def record_counters(per_mac_csv: str, per_mac_size: int, traffic_csv: str | None
     c["inst_per_mac"] = round(m["smsp__inst_executed.sum"] * 32 / macs, 3)
     c["alu_inst_per_mac"] = round(m["sm__inst_executed_pipe_alu.sum"] * 32 / macs, 3)
     if "sm__inst_executed_pipe_fma.sum" in m:
-        # fp32 instructions of this kernel's fast path are all packed fp32x2 (FMUL2 / FADD2 / FFMA2)
+        # FMA-pipe instructions of this kernel's fast path are all packed (FMUL2 on fp32 pairs, HADD2 on fp16 pairs)
         c["packed_fp_inst_per_mac"] = round(m["sm__inst_executed_pipe_fma.sum"] * 32 / macs, 3)
     if traffic_csv:
         t = metrics(traffic_csv)
@@ -823,9 +823,9 @@ def main() -> int:
         out = torch.empty(x.shape[0], S, device=dev)
         be.float_quantize_nearest_mm(x, y, out, x.shape[0], S, S, FMT["man_add"], FMT["exp_add"], FMT["man_mul"],
                                      FMT["exp_mul"], True, False, False, order=args.order)
-        # stats_init_kernel, two stats_kernel, mm_kernel, and for products of at least 2^33 MACs the exact_mm_kernel
+        # stats_init_kernel, stats_kernel, mm16_kernel, and for products of at least 2^33 MACs the exact_mm_kernel
         # launch that follows it (which finds nothing to do on these operands)
-        launches[0] += 4 + (1 if x.shape[0] * S * S >= 2 ** 33 else 0)
+        launches[0] += 3 + (1 if x.shape[0] * S * S >= 2 ** 33 else 0)
         return out
 
     def step():
@@ -834,7 +834,7 @@ def main() -> int:
         if world == 1:
             be.float_quantize_nearest_mm(a, b, c_full, S, S, S, FMT["man_add"], FMT["exp_add"], FMT["man_mul"],
                                          FMT["exp_mul"], True, False, False, order=args.order)
-            launches[0] += 4 + (1 if S ** 3 >= 2 ** 33 else 0)
+            launches[0] += 3 + (1 if S ** 3 >= 2 ** 33 else 0)
         else:
             sharded_float_mm(a, b, S, mm_rows, panels=panels, out=c_full)
 
