@@ -56,7 +56,8 @@ def record_counters(per_mac_csv: str, per_mac_size: int, traffic_csv: str | None
     """Rebuild profiles/mm_kernel_counters.json from ncu `--csv` logs of the GEMM kernel: `per_mac_csv` holds
     smsp__inst_executed.sum, sm__inst_executed_pipe_alu.sum, sm__inst_executed_pipe_fma.sum (and anything else asked for) of
     one mm16_kernel launch at M = N = K = `per_mac_size`; `traffic_csv` dram__bytes_read.sum / dram__bytes_write.sum of one
-    launch at 8192^3.  The hashes of the kernel sources as they are now are stored beside the numbers."""
+    launch at 8192^3.  The hashes of the kernel sources as they are now are stored beside the numbers; nothing of an earlier
+    capture is kept but the commands of the logs that were given, so that no figure of another kernel passes as one of this."""
     import csv
 
     def metrics(path):
@@ -76,9 +77,10 @@ def record_counters(per_mac_csv: str, per_mac_size: int, traffic_csv: str | None
     m = metrics(per_mac_csv)
     macs = float(per_mac_size) ** 3
     old = json.load(open(COUNTERS_PATH)) if os.path.exists(COUNTERS_PATH) else {}
-    c = dict(old)
-    c["kernel"] = m.pop("kernel", old.get("kernel"))
-    c["captured_at"] = note
+    c = {"kernel": m.pop("kernel"), "captured_at": note}
+    for key in ("command",) + (("command_traffic",) if traffic_csv else ()):
+        if key in old:
+            c[key] = old[key]
     c["metrics"] = {k: v for k, v in m.items()}
     c["metrics"]["macs"] = macs
     c["inst_per_mac"] = round(m["smsp__inst_executed.sum"] * 32 / macs, 3)
@@ -775,7 +777,7 @@ def main() -> int:
     if args.record_counters:
         rc = args.record_counters
         c = record_counters(rc[0], int(rc[1]), rc[2] if len(rc) > 2 else None,
-                            "float_mm %s^3 mul e5m2 / add e5m2 (per-MAC counters), 8192^3 (DRAM traffic)" % rc[1])
+                            "float_mm %s^3 mul e5m2 / add e5m2 (per-MAC counters)" % rc[1] + (", 8192^3 (DRAM traffic)" if len(rc) > 2 else ""))
         print(json.dumps(c))
         return 0
     if args.impl == "reference":
