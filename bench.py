@@ -10,8 +10,8 @@ all-gather of the C row blocks, so the total work is fixed ("strong" scaling).  
 rank 0.  Inputs (512 MiB) are larger than L2, so no flush is needed between iterations.
 
 `--impl reference` times the reference's own CPU implementation (oracle/_ref/quant_cpu, the unmodified
-reference extension, when it has been built; otherwise the C restatement in oracle/) on the host cores on a
-bounded row sample of the same problem.
+reference extension) on the host cores on a bounded row sample of the same problem, and says "unavailable" where that
+extension has not been built.
 """
 from __future__ import annotations
 
@@ -216,6 +216,12 @@ def cpu_baseline(rows_per_core: int = 1, cores: int | None = None) -> dict:
 def run_reference(args) -> int:
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    from oracle.build_ref import load_ref
+
+    if load_ref("quant_cpu") is None:      # cpu_baseline would time the oracle, this repository's own restatement
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU extension is not built here (oracle/build_ref.py "
+                                                              "needs the reference's sources)"}))
         return 0
     res = []
     for _ in range(max(0, args.warmup)):

@@ -40,3 +40,15 @@ def test_traffic_of_another_capture_is_dropped(bench, tmp_path, monkeypatch):
     traffic = log(tmp_path / "b.csv", [("dram__bytes_read.sum", "Gbyte", "1.5"), ("dram__bytes_write.sum", "Mbyte", "500")])
     c = bench.record_counters(per_mac, 32, traffic, "note")
     assert c["dram_bytes_per_launch_8192cubed"] == 2_000_000_000 and c["command_traffic"] == "t"
+
+
+def test_reference_arm_never_times_the_oracle(bench, monkeypatch, capsys):
+    import argparse
+
+    import oracle.build_ref
+
+    monkeypatch.setattr(oracle.build_ref, "load_ref", lambda name: None)
+    monkeypatch.setattr(bench, "cpu_baseline", lambda *a: pytest.fail("the oracle was timed as the reference"))
+    assert bench.run_reference(argparse.Namespace(gpus=1, steps=1, warmup=0)) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
