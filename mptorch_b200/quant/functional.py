@@ -283,6 +283,12 @@ def implicit_wgrad_eligible(formats) -> bool:
     return _float_nearest_spec(formats.grad_quant) is not None
 
 
+def _by_pointer(t: torch.Tensor) -> bool:
+    """A kernel that reads the tensor's memory may stand in for a torch operation on it: no graph is being recorded through it
+    (a backward pass with ``create_graph``), and it has memory of its own (a tensor under ``vmap`` or ``is_grads_batched`` has none)."""
+    return not (torch.is_grad_enabled() and t.requires_grad) and type(t) is torch.Tensor and torch._C._has_storage(t)
+
+
 class qconv2d_kernel(torch.autograd.Function):
     """Zero-padded 2-D convolution whose forward pass is one implicit GEMM per group on the NCHW input
     (``mpt_float_conv2d_nearest``): the unfolded input, nine times the input for a 3x3 kernel, is neither built nor
@@ -325,7 +331,7 @@ class qconv2d_kernel(torch.autograd.Function):
         c_out, cg, kh, kw = qweight.shape
         og = c_out // groups
         grad_scale = 0                # the implicit path is taken only without tensor scaling (implicit_conv_eligible)
-        grad_input, gws, gbs = None, [], []
+        grad_input, folded, gws, gbs = None, {}, [], []          # folded: what torch folded, by group
         implicit_w = ctx.needs_input_grad[1] and implicit_wgrad_eligible(f)
         # the implicit weight gradient runs beside the per-group input gradients (its quantizer is deterministic, so
         # the order of the calls does not matter to any random stream)
@@ -341,18 +347,17 @@ class qconv2d_kernel(torch.autograd.Function):
         for g in range(groups):
             go = grad_output[:, g * og:(g + 1) * og]
             go2 = go.reshape(n, og, -1).transpose(1, 2)
-            go2 = (_f32c(go2) if go2.dtype == torch.float32 else go2).reshape(-1, og)  # [N * L, og], as qlinear sees it
+            go2 = (_f32c(go2) if go2.dtype == torch.float32 and _by_pointer(go2) else go2).reshape(-1, og)  # [N * L, og], as qlinear sees it
             qgo = f.grad_quant(go2)
             w2 = qweight[g * og:(g + 1) * og].reshape(og, -1)
             if ctx.needs_input_grad[0]:
                 gc = torch.matmul(qgo, w2) if f.bwd_use_default_prec else mp_bmm(qgo, w2, formats=f, use_forward=False)
                 gc = f.grad_quant(gc)                                                # [N * L, K]
-                if grad_input is None:
+                if grad_input is None and _by_pointer(gc):
                     grad_input = torch.empty(n, c, h, w, device=gc.device, dtype=gc.dtype)
-                if not _be.fold_into(gc, grad_input, g * cg, cg, (kh, kw), stride, padding, dilation):
+                if not (_by_pointer(gc) and _be.fold_into(gc, grad_input, g * cg, cg, (kh, kw), stride, padding, dilation)):
                     gc = gc.view(n, -1, gc.shape[-1]).transpose(1, 2)                # [N, K, L]
-                    grad_input[:, g * cg:(g + 1) * cg] = torch.nn.functional.fold(gc, (h, w), (kh, kw), dilation=dilation,
-                                                                                  padding=padding, stride=stride)
+                    folded[g] = torch.nn.functional.fold(gc, (h, w), (kh, kw), dilation=dilation, padding=padding, stride=stride)
             if ctx.needs_input_grad[1] and not implicit_w:
                 cols = _conv_cols(qinput[:, g * cg:(g + 1) * cg], (kh, kw), dilation, padding, stride)
                 gw = (torch.matmul(qgo.transpose(-2, -1), cols) if f.bwd_use_default_prec
@@ -369,6 +374,8 @@ class qconv2d_kernel(torch.autograd.Function):
                             gb = qsum(qgo, dim=(0,), quant=make_quant_function(f.bwd_add, f.bwd_rnd, f.rbits_add))
                 gbs.append(f.grad_quant(gb.reshape(-1)))
         second.join(*gws)
+        if folded:
+            grad_input = torch.cat([folded[g] if g in folded else grad_input[:, g * cg:(g + 1) * cg] for g in range(groups)], dim=1)
         grad_weight = torch.cat(gws, dim=0) if gws else None
         grad_bias = torch.cat(gbs, dim=0) if gbs else None
         return grad_input, grad_weight, grad_bias, None, None, None, None, None
