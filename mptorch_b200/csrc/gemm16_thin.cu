@@ -156,16 +156,14 @@ __global__ void __launch_bounds__(TTHREADS + stagers(CONV), CONV == CONV_WGRAD ?
             {
                 const int row = tid >> 4, kc = (tid & 15) << 2;
                 const int gm = m0 + row, gk = k0 + kc;
-                int bytes = gm < p.M ? (p.K - gk) * 4 : 0;
-                bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
+                const int bytes = gm < p.M ? bytes16(p.K - gk) : 0;
                 cp_async16(as + row * TA_LD + kc, bytes ? A + (int64_t)gm * p.K + gk : A, bytes);
             }
 #pragma unroll
             for (int u = 0; u < TBK * TBN / 4 / TTHREADS; ++u) {
                 const int c = tid + u * TTHREADS, kr = c >> 3, nc = (c & 7) << 2;
                 const int gk = k0 + kr, gn = n0 + nc;
-                int bytes = gk < p.K ? (p.N - gn) * 4 : 0;
-                bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
+                const int bytes = gk < p.K ? bytes16(p.N - gn) : 0;
                 cp_async16(bs + kr * LDB + nc, bytes ? B + (int64_t)gk * p.N + gn : B, bytes);
             }
         } else {

@@ -242,8 +242,7 @@ __device__ __forceinline__ void load_tiles(const MmParams& p, const float* A, co
             if (kAChunks % THREADS != 0 && c >= kAChunks) break;
             const int row = c >> 3, kc = (c & 7) << 2;
             const int gm = m0 + row, gk = k0 + kc;
-            int bytes = (gm < p.M) ? (p.K - gk) * 4 : 0;
-            bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
+            const int bytes = gm < p.M ? bytes16(p.K - gk) : 0;
             const float* src = bytes ? A + (int64_t)gm * p.K + gk : A;
             cp_async16(As + row * AS_LD + kc, src, bytes);
         }
@@ -252,8 +251,7 @@ __device__ __forceinline__ void load_tiles(const MmParams& p, const float* A, co
             const int c = tid + u * THREADS;
             const int kr = c >> 4, nc = (c & 15) << 2;
             const int gk = k0 + kr, gn = n0 + nc;
-            int bytes = (gk < p.K) ? (p.N - gn) * 4 : 0;
-            bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
+            const int bytes = gk < p.K ? bytes16(p.N - gn) : 0;
             const float* src = bytes ? B + (int64_t)gk * p.N + gn : B;
             cp_async16(Bs + kr * BN + nc, src, bytes);
         }
