@@ -191,7 +191,9 @@ extern "C" int mpt_fold(const float* cols, float* out, int n_img, int channels, 
     const size_t smem = sizeof(float) * (size_t)g.rows * g.cols * (size_t)g.pitch;
     const bool dilated = (dil_h > 1 && KH > 1) || (dil_w > 1 && KW > 1);
     auto kern = vec ? (dilated ? fold_kernel<true, true> : fold_kernel<true, false>) : (dilated ? fold_kernel<false, true> : fold_kernel<false, false>);
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit belongs to the function on this device, not to the call: the same for every call, so that threads with different
+    // shapes leave one another's launches alone
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kFloats * sizeof(float)));
     if (e != cudaSuccess) { set_error("fold: cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MPT_ERR_CUDA; }
     kern<<<dim3((unsigned)tiles, (unsigned)gy, (unsigned)n_img), 256, smem, static_cast<cudaStream_t>(stream)>>>(cols, out, g);
     return check_launch("fold");

@@ -36,3 +36,33 @@ def test_shapes_left_to_torch():
     out = torch.empty(1, 1, 13, 13, device="cuda")
     assert not be.fold_into(torch.empty(1, 169, device="cuda"), out, 0, 1, (13, 13), (1, 1), (0, 0), (1, 1))
     assert not be.fold_into(torch.empty(169, 1, device="cuda").double(), out, 0, 1, (1, 1), (1, 1), (0, 0), (1, 1))
+
+
+def test_threads_folding_different_shapes():
+    """Several host threads, each on a stream of its own, with shapes that take the same kernel and 5 KB or 81 KB of shared
+    memory: no thread's launch depends on what another one has set."""
+    import threading
+
+    from mptorch_b200 import backend as be
+
+    failures = []
+
+    def work(c, size, k, pad):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                cols = torch.randn(size * size, c * k * k, device="cuda")
+                out = torch.empty(1, c, size, size, device="cuda")
+                for _ in range(3000):
+                    assert be.fold_into(cols, out, 0, c, (k, k), (1, 1), (pad, pad), (1, 1))
+                want = torch.nn.functional.fold(cols.view(1, size * size, -1).transpose(1, 2), (size, size), (k, k), padding=pad)
+                assert torch.equal(out, want)
+        except Exception as e:
+            failures.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=a) for a in ((16, 14, 3, 1), (16, 8, 1, 0)) * 3]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[0]
