@@ -141,6 +141,10 @@ MPT_API int mpt_superfp_quantize_nearest(const float *in, float *out, int64_t n,
  * path only. */
 MPT_API size_t mpt_mm_workspace_bytes(int64_t batch);
 
+/* No counterpart in the reference.  Output rows per tile (8, 64 or 128) that a product with e5m10, e8m7, e5m2 or e4m3 sums takes
+ * on the current device: the kernels differ by tile height, and tests ask for it so that each one is met. */
+MPT_API int mpt_mm16_tile_rows(int64_t batch, int M, int N, int compensated);
+
 /* replaces float_quantize_nearest_mm and _bmm (pybind_cuda.cpp:123,140 -> quant.cu:335,362 ->
  * fp_kernel.cu:174-245 -> mm_kernel.h:19-132) and their CPU twins (quant_cpu/mm_kernel.h:9-34).
  *   C[b] = A[b] x B[b],  A: [batch, M, K], B: [batch, K, N], C: [batch, M, N]

@@ -71,6 +71,7 @@ def lib() -> C.CDLL:
             "mpt_float_mm_nearest_piece": [p, p, p, i64] + [i32] * 12 + [p, sz, p],
             "mpt_copy_columns_async": [p, sz, p, sz, sz, sz, p],
             "mpt_transpose_last2": [p, p, i64, i64, i64, p],
+            "mpt_mm16_tile_rows": [i64, i32, i32, i32],
             "mpt_fold": [p, p] + [i32] * 12 + [i64, p],
             "mpt_float_mm_nearest_fma": [p, p, p, i64, i32, i32, i32, i32, i32, i32, i32, i32, i32, p, sz, p],
             "mpt_float_mm_stochastic": [p, p, p, i64, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, u64, p, sz, p],

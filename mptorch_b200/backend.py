@@ -268,6 +268,11 @@ def float_mm_nearest_piece(a, b, c, man_add, exp_add, man_mul, exp_mul, subnorma
              stream_ptr(a.device))
 
 
+def mm16_tile_rows(M: int, N: int, batch: int = 1, compensated: bool = False) -> int:
+    """Output rows per tile (8, 64 or 128) of a product on 16-bit sums on the current device (``mpt_mm16_tile_rows``)."""
+    return _cabi.lib().mpt_mm16_tile_rows(batch, M, N, int(bool(compensated)))
+
+
 def transpose_last2(x):
     """A dense copy of ``x.transpose(-2, -1)`` for a contiguous float32 CUDA tensor with at least two dimensions, or None
     when the kernel's grid limits do not admit the shape (the caller then lets torch copy)."""

@@ -330,6 +330,11 @@ size_t mpt_mm_workspace_bytes(int64_t batch) {
     return (need + 255) & ~(size_t)255;
 }
 
+int mpt_mm16_tile_rows(int64_t batch, int M, int N, int compensated) {
+    const Tile16 t = pick_tile16(M, N, batch, !compensated);
+    return t == TILE16_THIN ? 8 : t == TILE16_MID ? 64 : BM;
+}
+
 int mpt_float_mm_nearest(const float* a, const float* b, float* c, int64_t batch, int M, int N, int K, int man_add,
                          int exp_add, int man_mul, int exp_mul, int subnormals, int saturate, int compensated,
                          int order, void* workspace, size_t workspace_bytes, void* stream) {

@@ -26,8 +26,9 @@ def check(be, oracle, a, b, what, **kw):
     assert same_bits(got, want), f"{what} {kw}: " + mismatch_report(got, want)
 
 
-# (batch, M, K, N): single elements, one short of and one past a group of 8, a slab of 32 and both tile heights; 160 batch
-# entries are more tiles than SMs, which selects the 128-row tiles
+# (batch, M, K, N): single elements, one short of and one past a group of 8, a slab of 32 and the tiles' edges.  The rule sends
+# the plain and fused forms of all of them to tiles of 8 rows and compensated sums to tiles of 64; the other tile heights
+# are further down.
 SHAPES = [(1, 1, 1, 1), (1, 15, 7, 63), (1, 17, 9, 65), (1, 16, 32, 64), (1, 33, 33, 4), (160, 3, 31, 5), (160, 5, 8, 66), (2, 129, 64, 68)]
 
 
@@ -96,4 +97,124 @@ def test_continuing_from_sums_outside_the_format(be, oracle, fmts):
                               False, be.MM_PIECE_FROM_C, order="cuda")
     inner = cpu_mm(oracle, a, b, fadd, fmul)             # one group of eight from zero, folded into +0
     want = oracle.float_quantize((c0 + inner).astype(np.float32), fadd[1], fadd[0], "nearest", True, False)
+    assert same_bits(c.cpu().numpy(), want), mismatch_report(c.cpu().numpy(), want)
+
+
+# ---- every tile height ------------------------------------------------------------------------------------------------
+# Results that the rule sends to tiles of 8, 64 and 128 rows on a GPU of 148 SMs (`tile` is asked of the library, so that a rule
+# that moves is noticed), each ragged in both directions and with K short of and past whole groups and slabs.
+BATCHED = {8: (40, 21, 41, 37), 64: (140, 63, 41, 61), 128: (140, 113, 41, 50)}
+# compensated sums have no tiles of 8 rows
+COMPENSATED = {64: (40, 61, 21, 63), 128: (140, 113, 21, 50)}
+# tiles inside the matrix beside ragged ones, with 16-byte copies (K and N multiples of 4) and without; three slabs of 32, two of 64
+LARGE = {8: [(252, 72, 100), (67, 73, 99)], 64: [(700, 72, 700), (707, 73, 701)], 128: [(700, 72, 1028), (701, 73, 1027)]}
+
+
+def tile(be, M, N, batch=1, comp=False):
+    return be.mm16_tile_rows(M, N, batch, comp)
+
+
+def scaled_batch(rng, B, M, K, N):
+    """Batch entries in turn: in range, below the smallest normal value, sums that flush, past the formats' range, with
+    infinities and NaN, zeros of both signs with a plan and (an infinity among them) without, exact cancellations without."""
+    a = rng.standard_normal((B, M, K)).astype(np.float32)
+    b = rng.standard_normal((B, K, N)).astype(np.float32)
+    for i, scale in enumerate((1.0, 2.0 ** -6, 2.0 ** -13, 24.0)):
+        a[i::8] *= np.float32(scale)
+    a[4::8][rng.random(a[4::8].shape) < 0.01] = np.inf
+    b[4::8][rng.random(b[4::8].shape) < 0.01] = np.nan
+    for i in (5, 6):
+        a[i::8] = np.where(rng.random(a[i::8].shape) < 0.9, np.float32(-0.0), a[i::8])
+    a[7::8, :, 1::2], b[7::8, 1::2] = -a[7::8, :, :K - 1:2], b[7::8, :K - 1:2]
+    a[6::8, M // 2, K // 2] = a[7::8, M // 3, K // 2] = np.inf
+    a[2::8, 0, 0], b[2::8, 0, 0] = 2.0 ** -80, 2.0 ** -60      # 8-bit exponents: a product that is an fp32 denormal
+    return a, b
+
+
+@pytest.mark.parametrize("rows", [8, 64, 128])
+@pytest.mark.parametrize("sub", [True, False])
+@pytest.mark.parametrize("fmts", PAIRS)
+def test_each_tile_height(be, oracle, fmts, sub, rows):
+    fadd, fmul = fmts
+    rng = np.random.default_rng(100 * fadd[1] + fmul[1] + rows)
+    B, M, K, N = BATCHED[rows]
+    assert tile(be, M, N, B) == rows
+    a, b = scaled_batch(rng, B, M, K, N)
+    for order in ("cuda", "seq"):
+        for fma in (False, True):
+            check(be, oracle, a, b, BATCHED[rows], fadd=fadd, fmul=fmul, sub=sub, fma=fma, order=order)
+    check(be, oracle, a, b, BATCHED[rows], fadd=fadd, fmul=fmul, sub=sub, sat=True)
+    if rows in COMPENSATED:
+        B, M, K, N = COMPENSATED[rows]
+        assert tile(be, M, N, B, True) == rows
+        a, b = scaled_batch(rng, B, M, K, N)
+        for fma in (False, True):
+            check(be, oracle, a, b, COMPENSATED[rows], fadd=fadd, fmul=fmul, sub=sub, fma=fma, comp=True)
+
+
+@pytest.mark.parametrize("rows", [8, 64, 128])
+@pytest.mark.parametrize("sub", [True, False])
+@pytest.mark.parametrize("fmts", PAIRS)
+def test_tiles_inside_the_matrix(be, oracle, fmts, sub, rows):
+    fadd, fmul = fmts
+    rng = np.random.default_rng(10 * fadd[1] + fmul[1] + rows)
+    for M, K, N in LARGE[rows]:
+        assert tile(be, M, N) == rows
+        # rows of every size of sum: in range, flushing, and (e4m3, e5m2) past the limit of the range check in the long run
+        a = rng.standard_normal((M, K)).astype(np.float32) * np.float32(2.0) ** rng.integers(-9, 1, (M, 1)).astype(np.float32)
+        b = rng.standard_normal((K, N)).astype(np.float32)
+        for order in ("cuda", "seq"):
+            check(be, oracle, a, b, (M, K, N), fadd=fadd, fmul=fmul, sub=sub, order=order)
+        check(be, oracle, a, b, (M, K, N), fadd=fadd, fmul=fmul, sub=sub, fma=True)
+
+
+def continued(oracle, a, b, c, fadd, fmul, sub, order):
+    """The definition of a last piece: the product's steps from what C holds, one rounded operation at a time."""
+    def q(x, fmt):
+        return oracle.float_quantize(np.ascontiguousarray(x, np.float32), fmt[1], fmt[0], "nearest", sub, False)
+
+    K = a.shape[1]
+    steps = [q(a[:, k, None] * b[None, k, :], fmul) for k in range(K)]
+    acc = c.copy()
+    if order == "seq":
+        for p in steps:
+            acc = q(acc + p, fadd)
+        return acc
+    for k0 in range(0, K + 8 - K % 8, 8):                 # the order's last group is of zeros where K is a multiple of eight
+        inner = np.zeros_like(c)
+        for p in steps[k0:k0 + 8]:
+            inner = q(inner + p, fadd)
+        for _ in range(max(k0 + 8 - max(K, k0), 0)):
+            inner = q(inner + np.float32(0.0), fadd)
+        acc = q(acc + inner, fadd)
+    return acc
+
+
+@pytest.mark.parametrize("rows", [8, 64, 128])
+@pytest.mark.parametrize("order", ["cuda", "seq"])
+@pytest.mark.parametrize("sub,planned", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("fmts", PAIRS)
+def test_continuing_on_each_tile_height(be, oracle, fmts, sub, planned, order, rows):
+    """Pieces that continue from sums outside the format (32-bit values, zeros of both signs, infinities, NaN) and from rounded
+    ones; with operands that pass the range check (where the formats let them) and with an infinity, which never does."""
+    fadd, fmul = fmts
+    M, K, N = LARGE[rows][0]
+    K = K if rows == 8 else 40                            # two slabs of either kernel
+    rng = np.random.default_rng(17 + rows)
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    b = rng.standard_normal((K, N)).astype(np.float32)
+    a[1] = -0.0
+    if not planned:
+        a[M // 2, K - 2] = np.inf
+    c0 = rng.standard_normal((M, N)).astype(np.float32)
+    c0[rng.random(c0.shape) < 0.05] = -0.0
+    c0[rng.random(c0.shape) < 0.001] = np.inf
+    c0[rng.random(c0.shape) < 0.001] = np.nan
+    c0[: M // 2] = oracle.float_quantize(c0[: M // 2], fadd[1], fadd[0], "nearest", sub, False)
+    c0[1] = -0.0
+    c = torch.from_numpy(c0.copy()).cuda()
+    be.float_mm_nearest_piece(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), c, fadd[1], fadd[0], fmul[1], fmul[0], sub, False,
+                              False, be.MM_PIECE_FROM_C, order=order)
+    with np.errstate(all="ignore"):
+        want = continued(oracle, a, b, c0, fadd, fmul, sub, order)
     assert same_bits(c.cpu().numpy(), want), mismatch_report(c.cpu().numpy(), want)
