@@ -291,14 +291,17 @@ def fold_into(cols, out, first_channel, channels, kernel_size, stride, padding, 
     """Channels first_channel .. first_channel + channels - 1 of ``out`` [N, C, H, W] = the folded ``cols``
     [N * OH * OW, channels * KH * KW] (``mpt_fold``); False, with nothing done, where the kernel does not take the tensors or
     the shape (the caller then lets torch fold)."""
-    (kh, kw), n = kernel_size, out.shape[0]
+    (kh, kw), (n, _, h, w) = kernel_size, out.shape
+    oh, ow = ((e + 2 * p - d * (k - 1) - 1) // s + 1 for e, k, s, p, d in zip((h, w), kernel_size, stride, padding, dilation))
+    if cols.shape != (n * oh * ow, channels * kh * kw) or first_channel < 0 or first_channel + channels > out.shape[1]:
+        raise ValueError("fold_into: cols %s does not hold the %d x %d positions of %d channels from %d on of %s"
+                         % (tuple(cols.shape), oh, ow, channels, first_channel, tuple(out.shape)))
     reach = [(k - 1) * d // s + 1 for k, d, s in zip(kernel_size, dilation, stride)]
     for t in (cols, out):
         if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
             return False
     if n > 65535 or channels > 65535 or reach[0] * reach[1] * (kh * kw + 1) > 24576 or cols.device != out.device:
         return False
-    h, w = out.shape[2:]
     with torch.cuda.device(out.device):
         call("mpt_fold", ptr(cols), out.data_ptr() + 4 * first_channel * h * w, n, channels, h, w, kh, kw, stride[0], stride[1],
              padding[0], padding[1], dilation[0], dilation[1], out.shape[1] * h * w, stream_ptr(out.device))
