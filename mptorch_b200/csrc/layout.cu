@@ -154,8 +154,13 @@ extern "C" int mpt_fold(const float* cols, float* out, int n_img, int channels, 
     if (n_img == 0 || channels == 0 || H == 0 || W == 0) return MPT_OK;
     FoldGeom g;
     g.H = H; g.W = W; g.KH = KH; g.KW = KW; g.sh = stride_h; g.sw = stride_w; g.ph = pad_h; g.pw = pad_w; g.dh = dil_h; g.dw = dil_w;
-    const int64_t span_h = (int64_t)H + 2 * pad_h - (int64_t)dil_h * (KH - 1) - 1, span_w = (int64_t)W + 2 * pad_w - (int64_t)dil_w * (KW - 1) - 1;
+    const int64_t span_h = H + 2 * (int64_t)pad_h - (int64_t)dil_h * (KH - 1) - 1, span_w = W + 2 * (int64_t)pad_w - (int64_t)dil_w * (KW - 1) - 1;
     MPT_REQUIRE(span_h >= 0 && span_w >= 0, "fold: no output position");
+    // what the kernel works out about positions, reaches and kernel rows is 32 bits wide
+    const auto fits = [](int64_t e, int64_t k, int64_t s, int64_t p, int64_t d, int64_t span) {
+        return e + p + s - 2 <= 0x7FFFFFFF && (k - 1) * d <= 0x7FFFFFFF && span / s < 0x7FFFFFFF;
+    };
+    MPT_REQUIRE(fits(H, KH, stride_h, pad_h, dil_h, span_h) && fits(W, KW, stride_w, pad_w, dil_w, span_w), "fold: padded image or stride too large");
     g.OH = (int)(span_h / stride_h) + 1; g.OW = (int)(span_w / stride_w) + 1;
     g.channels = channels; g.out_image_stride = out_image_stride;
     MPT_REQUIRE(cols && out && out_image_stride >= (int64_t)channels * H * W, "fold: bad arguments");
