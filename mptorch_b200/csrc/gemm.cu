@@ -272,6 +272,8 @@ int check_mm_args(const char* who, const float* a, const float* b, float* c, int
     MPT_REQUIRE(batch >= 0 && M >= 0 && N >= 0 && K >= 0, "%s: negative dimension", who);
     MPT_REQUIRE(batch <= 65535, "%s: batch %lld exceeds 65535", who, (long long)batch);
     MPT_REQUIRE(((int64_t)M + BM - 1) / BM <= 65535, "%s: M=%d too large", who, M);
+    // the kernels number the columns and steps of a tile that hangs over the edge, and those of the slabs fetched ahead, in 32 bits
+    MPT_REQUIRE(N <= 0x7FFFFFFF - 256 && K <= 0x7FFFFFFF - 256, "%s: N=%d or K=%d too large", who, N, K);
     const bool empty = batch == 0 || M == 0 || N == 0;
     MPT_REQUIRE(empty || (c && (K == 0 || (a && b))), "%s: null pointer", who);
     return MPT_OK;

@@ -30,3 +30,11 @@ def test_fold_of_images_past_32_bits(size, kernel, stride, pad, dil):
     p = C.c_void_p(16)
     assert refused(fold(p, p, 1, 1, size, 1, kernel, 1, stride, 1, pad, 0, dil, 1, size, None))
     assert refused(fold(p, p, 1, 1, 1, size, 1, kernel, 1, stride, 0, pad, 1, dil, size, None))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 0x7FFFFFFF, 1), (1, 0x7FFFFFFF - 255, 4), (1, 1, 0x7FFFFFFF), (4, 8, 0x7FFFFFFF - 100)])
+def test_products_past_32_bits(M, N, K):
+    from mptorch_b200 import _cabi
+
+    p = C.c_void_p(16)
+    assert refused(_cabi.lib().mpt_float_mm_nearest(p, p, p, 1, M, N, K, 10, 5, 3, 4, 1, 0, 0, 1, p, 256, None))
