@@ -1,5 +1,5 @@
 // Column chains with 16-bit running sums: layernorm parameter gradients and mpt_qsum_rows where the accumulation format is
-// e5m10 or e8m7 (colsum_kernel in reduce.cu is the general form), and the same sums over few rows in any format.
+// e5m10 or e8m7 (colsum_kernel in reduce.cu is the general form), and column sums over many columns in any format.
 //
 // out[c] = the running sum acc = Q(acc + v[r]) over the rows in order.  The chain is serial by definition, so its time is the
 // rows times the latency of one rounded addition.  The value after each step is a binary16 (bfloat16) value, and the
@@ -245,8 +245,20 @@ int launch_chain16(int mode, const float* in, const float* gout, const float* me
     return r16 ? run(chain16_kernel<0, false, R16_F16, false>) : run(chain16_kernel<0, false, R16_ANY, false>);
 }
 
-// Where one thread per column beats a chain warp per eight columns: the columns alone fill the GPU's threads.
-bool wide_colsum_ok(const RowGeom& g) { return g.inner == 1 && g.channel >= 32768; }
+// Column sums (mode 1): which kernel?  Measured in us, inputs not in L2, general chain against the 16-bit chain:
+//   e5m10:                 8192 columns x 1024 rows 38, 30; 12,288 x 1024: 42, 41 (e8m7 46); 16,384 x 1024: 44, 51; x 128: 10, 13
+//   without subnormals:    16,384 x 128 rows 34, 37 (e8m7 12); x 256: 64, 58; x 1024: 245, 99 (e8m7 57)
+// and the general chain against a thread per column (inputs in L2 where they fit):
+//   e5m10:                 32,768 x 128 rows 15, 10; x 1024: 76, 107; 65,536 x 1024: 123, 113; 786,432 x 8: 50, 10
+//   without subnormals:    32,768 x 1024 rows 469, 275; fp32 sums: 197, 161
+// The 16-bit chain's short steps pay while columns are too few to fill the SMs.  A thread per column wants enough columns to
+// cover the trips to memory, or few rows; against the general chain's exact casters it wins at any number of rows.
+bool chain16_wins(const RowGeom& g, const Caster& acc) {
+    return g.channel <= 8192 || (!acc.any.fp.sub && g.rows >= (acc.any.fp.exp == 8 ? 32 : 256));
+}
+bool wide_colsum_ok(const RowGeom& g, const SeqAdder& seq) {
+    return g.inner == 1 && (g.channel >= 65536 || (g.channel >= 32768 && (g.rows <= 128 || !seq.chain_ok)));
+}
 int launch_wide_colsum(const float* in, float* out, const RowGeom& g, const SeqAdder& seq, cudaStream_t st, const char* who) {
     wide_colsum_kernel<<<(unsigned)((g.channel + 255) / 256), 256, 0, st>>>(in, out, g, seq);
     return check_launch(who);

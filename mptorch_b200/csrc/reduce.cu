@@ -265,8 +265,8 @@ __global__ void __launch_bounds__(chain_threads(MODE)) colsum_kernel(const float
 template <int MODE>
 int launch_colsum(const float* in, const float* gout, const float* mean, const float* rstd, float* out0, float* out1, const RowGeom& g,
                   const Caster& facc, const Caster& fmul, const SeqAdder& seq, cudaStream_t st, const char* who) {
-    if (MODE == 1 && wide_colsum_ok(g)) return launch_wide_colsum(in, out0, g, seq, st, who);
-    if (chain16_ok(facc)) return launch_chain16(MODE, in, gout, mean, rstd, out0, out1, g, facc, fmul, st, who);
+    if (MODE == 1 && wide_colsum_ok(g, seq)) return launch_wide_colsum(in, out0, g, seq, st, who);
+    if (chain16_ok(facc) && (MODE == 0 || chain16_wins(g, facc))) return launch_chain16(MODE, in, gout, mean, rstd, out0, out1, g, facc, fmul, st, who);
     const size_t smem = chain_smem_bytes(MODE);
     const bool line = MODE == 0 && facc.use_fast && fmul.use_fast && facc.any.fp.exp < 8 && fmul.any.fp.exp < 8;
     auto kern = line ? colsum_kernel<MODE, true> : colsum_kernel<MODE, false>;

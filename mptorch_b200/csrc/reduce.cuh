@@ -520,7 +520,8 @@ void launch_layernorm_bwd_rows(const float* in, const float* grad_out, const flo
 bool chain16_ok(const Caster& acc);
 int launch_chain16(int mode, const float* in, const float* gout, const float* mean, const float* rstd, float* out0, float* out1,
                    const RowGeom& g, const Caster& facc, const Caster& fmul, cudaStream_t st, const char* who);
-bool wide_colsum_ok(const RowGeom& g);
+bool chain16_wins(const RowGeom& g, const Caster& acc);
+bool wide_colsum_ok(const RowGeom& g, const SeqAdder& seq);
 int launch_wide_colsum(const float* in, float* out, const RowGeom& g, const SeqAdder& seq, cudaStream_t st, const char* who);
 
 }  // namespace mpt

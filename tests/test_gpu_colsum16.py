@@ -62,6 +62,23 @@ def test_qsum_of_few_rows_and_many_columns(oracle, fmt, rows):
         assert same_bits(got, want), f"{name}: " + mismatch_report(got, want)
 
 
+@pytest.mark.parametrize("rows,cols", [(40, 8192), (40, 8193), (31, 8200), (32, 8200), (255, 8200), (256, 8200), (128, 32768), (129, 32768),
+                                       (129, 65535), (129, 65536)])
+@pytest.mark.parametrize("sub", [True, False])
+@pytest.mark.parametrize("fmt", FORMATS + [(4, 3), (8, 23)])
+def test_qsum_on_both_sides_of_each_rule(oracle, fmt, sub, rows, cols):
+    """The kernel changes with the columns, the rows and the format; the sums do not."""
+    import mptorch_b200.quant as q
+
+    e, m = fmt
+    x = np.random.default_rng(rows).standard_normal((rows, cols)).astype(np.float32)
+    x[:, ::7] *= np.float32(2.0 ** -13)
+    x[:, 1::7] *= np.float32(9000.0)
+    x[rows // 2, 2::7] = np.inf
+    got, want = q.qsum_rows(dev(x), e, m, sub, False).cpu().numpy(), oracle.qsum_rows(x, m, e, sub, False)
+    assert same_bits(got, want), mismatch_report(got, want)
+
+
 @pytest.mark.parametrize("acc,mul", [((5, 10), (5, 10)), ((8, 7), (8, 7)), ((5, 10), (4, 3)), ((8, 7), (5, 10))])
 @pytest.mark.parametrize("sub", [True, False])
 @pytest.mark.parametrize("sat", [True, False])
