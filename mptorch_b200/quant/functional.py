@@ -283,6 +283,13 @@ def implicit_wgrad_eligible(formats) -> bool:
     return _float_nearest_spec(formats.grad_quant) is not None
 
 
+# Elements from which the transposing copy and the fold kernel repay their call in a backward pass of plain torch arithmetic, which
+# is host-bound below (a call from Python costs about 10 us more there than a torch operation).  Copy of the output
+# gradient: 18.6 us at any size against torch's 9 up to 0.8 M elements, 16.5 at 3.2 M and the bus beyond.  Fold of the
+# unfolded gradient: 15-20 us against torch's 25 at 0.5 M, 37 against 135 at 7.2 M; small layers lost 10-20 us of 300.
+_TRANSPOSE_FROM, _FOLD_FROM = 1 << 22, 1 << 19
+
+
 def _by_pointer(t: torch.Tensor) -> bool:
     """A kernel that reads the tensor's memory may stand in for a torch operation on it: no graph is being recorded through it
     (a backward pass with ``create_graph``), and it has memory of its own (a tensor under ``vmap`` or ``is_grads_batched`` has none)."""
@@ -347,15 +354,17 @@ class qconv2d_kernel(torch.autograd.Function):
         for g in range(groups):
             go = grad_output[:, g * og:(g + 1) * og]
             go2 = go.reshape(n, og, -1).transpose(1, 2)
-            go2 = (_f32c(go2) if go2.dtype == torch.float32 and _by_pointer(go2) else go2).reshape(-1, og)  # [N * L, og], as qlinear sees it
+            by_kernel = go2.dtype == torch.float32 and go2.numel() >= _TRANSPOSE_FROM and _by_pointer(go2)
+            go2 = (_f32c(go2) if by_kernel else go2).reshape(-1, og)                 # [N * L, og], as qlinear sees it
             qgo = f.grad_quant(go2)
             w2 = qweight[g * og:(g + 1) * og].reshape(og, -1)
             if ctx.needs_input_grad[0]:
                 gc = torch.matmul(qgo, w2) if f.bwd_use_default_prec else mp_bmm(qgo, w2, formats=f, use_forward=False)
                 gc = f.grad_quant(gc)                                                # [N * L, K]
-                if grad_input is None and _by_pointer(gc):
+                by_kernel = _by_pointer(gc) and (gc.numel() >= _FOLD_FROM or not f.bwd_use_default_prec)
+                if grad_input is None and by_kernel:
                     grad_input = torch.empty(n, c, h, w, device=gc.device, dtype=gc.dtype)
-                if not (_by_pointer(gc) and _be.fold_into(gc, grad_input, g * cg, cg, (kh, kw), stride, padding, dilation)):
+                if not (by_kernel and _be.fold_into(gc, grad_input, g * cg, cg, (kh, kw), stride, padding, dilation)):
                     gc = gc.view(n, -1, gc.shape[-1]).transpose(1, 2)                # [N, K, L]
                     folded[g] = torch.nn.functional.fold(gc, (h, w), (kh, kw), dilation=dilation, padding=padding, stride=stride)
             if ctx.needs_input_grad[1] and not implicit_w:

@@ -94,12 +94,23 @@ def test_batched_gradients_on_the_gpu():
 
 
 @pytest.mark.gpu
-def test_ordinary_backward_takes_the_fold_kernel(monkeypatch):
+@pytest.mark.parametrize("size,low,kernel", [(7, False, False), (7, True, True), (64, False, True)])
+def test_ordinary_backward_takes_the_fold_kernel(monkeypatch, size, low, kernel):
+    """Where the backward pass has its own formats, and in the default one from the size on that repays the call."""
     import mptorch_b200.backend as be
+    import mptorch_b200.quant as q
+    from mptorch_b200 import FloatingPoint
 
     took = []
     real = be.fold_into
     monkeypatch.setattr(be, "fold_into", lambda *a: (took.append(real(*a)), took[-1])[1])
-    conv, x = make(CASES[1], "cuda")
-    conv(x).sum().backward()
-    assert took == [True, True]
+    mac = (FloatingPoint(5, 10, True, False), FloatingPoint(4, 3, True, False))
+    conv = q.QConv2d(16, 6, 3, q.QAffineFormats(fwd_mac=mac, **({"bwd_mac": mac} if low else {})), padding=1, groups=2).cuda()
+    x = torch.randn(2, 16, size, size, device="cuda", requires_grad=True)
+    y = conv(x)
+    g = torch.randn_like(y)
+    y.backward(g)
+    assert took == ([True, True] if kernel else [])
+    if not low:
+        want = torch.nn.grad.conv2d_input(x.shape, conv.weight, g, padding=1, groups=2)
+        assert (x.grad - want).norm() <= 1e-5 * want.norm()
