@@ -354,7 +354,8 @@ class qconv2d_kernel(torch.autograd.Function):
         for g in range(groups):
             go = grad_output[:, g * og:(g + 1) * og]
             go2 = go.reshape(n, og, -1).transpose(1, 2)
-            by_kernel = go2.dtype == torch.float32 and go2.numel() >= _TRANSPOSE_FROM and _by_pointer(go2)
+            by_kernel = (go2.dtype == torch.float32 and (go2.numel() >= _TRANSPOSE_FROM or not f.bwd_use_default_prec)
+                         and _by_pointer(go2))
             go2 = (_f32c(go2) if by_kernel else go2).reshape(-1, og)                 # [N * L, og], as qlinear sees it
             qgo = f.grad_quant(go2)
             w2 = qweight[g * og:(g + 1) * og].reshape(og, -1)
