@@ -298,6 +298,151 @@ __device__ __forceinline__ void negate_all(float (&f)[TM][TN]) {      // zeros b
         for (int j = 0; j < TN; ++j) f[i][j] = add_rn(0.0f, -f[i][j]);
 }
 
+// ---- entries without a plan ----------------------------------------------------------------------------------------------
+// Operands that rule the range check out (an infinity or NaN, products or sums that may pass a format's range, as N(0,1) data in
+// e4m3 sums do) take 32-bit sums and the FP-pipe rounding.  Bound: the ALU pipe.  A rounding in its whole-domain form costs
+// nine ALU operations, of which six only find overflow; so a group is rounded without them, the largest magnitude that went
+// in is kept, and rows of a group with one that the short form does not cover are done again in the whole-domain form.  1024^3 with
+// one infinity, e5m10: 1.00 ms against 5.9 with the whole-domain form in a call per step (2.0 on 16-row tiles); 768 x 1024 x 768
+// e4m3 sums of N(0,1): 0.45 against 3.0 (1.2 on 16-row tiles).
+struct ShortRn {
+    FastRn r;
+    uint32_t lim;             // smallest |x| pattern that is not covered
+    __device__ __forceinline__ static ShortRn make(const FullRn& f) { return ShortRn{f.fast, min(f.ovf_from, f.exact_from)}; }
+};
+// What went into a rounding: the largest |x| pattern and, for 8-bit exponents, the smallest (|x| pattern - 1), where fp32
+// denormals show, which those formats treat specially.  Zero is covered: a sum from +0 is never -0, and the sign of a
+// product that is zero does not matter to it.  A fused sum can underflow to -0, so there zero counts as a denormal.
+template <bool EIGHT, bool FMA> struct Seen {
+    uint32_t top = 0u, low = 0xFFFFFFFFu;
+    __device__ __forceinline__ float round(const ShortRn& q, float x) {
+        const uint32_t a = __float_as_uint(x) & 0x7FFFFFFFu;
+        top = max(top, a);
+        if (EIGHT) low = min(low, FMA ? a : a - 1u);
+        return q.r(x);
+    }
+    __device__ __forceinline__ bool covered(const ShortRn& q) const { return top < q.lim && (!EIGHT || low >= (FMA ? 0x00800000u : 0x007FFFFFu)); }
+};
+// `nk` steps of R rows (`row` floats apart in the A slab) by C columns of outputs.  False: the sums are not to be used.
+template <bool FMA, bool EIGHT, int R, int C>
+__device__ __forceinline__ bool short_steps(float (&acc)[R][C], const float* a, int row, const float* b, int ldb, int nk, const ShortRn& qa,
+                                            const ShortRn& qm) {
+    Seen<EIGHT, FMA> sa, sm;
+#pragma unroll 1
+    for (int k = 0; k < nk; ++k) {
+        float bv[C];
+#pragma unroll
+        for (int j = 0; j < C; j += 2) { const float2 t = *reinterpret_cast<const float2*>(b + k * ldb + j); bv[j] = t.x; bv[j + 1] = t.y; }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float av = a[i * row + k];
+#pragma unroll
+            for (int j = 0; j < C; ++j)
+                acc[i][j] = sa.round(qa, FMA ? fma_rn(av, bv[j], acc[i][j]) : add_rn(acc[i][j], sm.round(qm, mul_rn(av, bv[j]))));
+        }
+    }
+    return sa.covered(qa) && (FMA || sm.covered(qm));
+}
+
+// The thread's outputs of one batch entry without a plan.  EIGHT: a format has 8 exponent bits.
+template <int ALGO, bool FMA, bool EIGHT>
+__device__ __forceinline__ void exact_tile16(const MmParams* pp, float* smem, int64_t batch, int m0, int n0) {
+    const MmParams& p = *pp;
+    float* As = smem;
+    float* Bs = smem + STAGES * SMEM_A;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const float* A = p.a + batch * p.stride_a;
+    const float* B = p.b + batch * p.stride_b;
+    float* C = p.c + batch * p.stride_c;
+    const int ksteps = (ALGO == ALGO_SEQ || (p.resume & MM_MORE)) ? p.K : p.K + 8 - p.K % 8;
+    const int ntiles = (ksteps + BK - 1) / BK;
+    const ShortRn qa = ShortRn::make(p.wadd), qm = ShortRn::make(p.wmul);
+    constexpr int R = 2;                 // rows at once: eight independent chains
+
+    float acc[TM][TN], outer[TM][TN];    // running (inner) sums; outer sums of the CUDA order
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = outer[i][j] = 0.0f;
+    if (p.resume & MM_FROM_C) {
+        if (ALGO == ALGO_TILE8) load_c(p, C, m0, n0, ty, tx, outer); else load_c(p, C, m0, n0, ty, tx, acc);
+    }
+    auto stage = [&](int s, int k0) {
+        if (p.vec) load_tiles<true>(p, A, B, As + s * SMEM_A, Bs + s * SMEM_B, m0, n0, k0, tid);
+        else load_tiles<false>(p, A, B, As + s * SMEM_A, Bs + s * SMEM_B, m0, n0, k0, tid);
+    };
+#pragma unroll 1
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < ntiles) stage(s, s * BK);
+        cp_async_commit();
+    }
+    // running sums of 8-bit-exponent formats that are -0 (continued from one, or flushed to one where there are no subnormals) keep
+    // the sign, which the short form does not
+    const bool never = EIGHT && ((p.resume & MM_FROM_C) || !p.whole_ok);
+    uint32_t missed = 0u;                // bit i: rows i of the thread were not covered last time; tried again every eighth group
+#pragma unroll 1
+    for (int t = 0; t < ntiles; ++t) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();
+        const int nt = t + STAGES - 1;
+        if (nt < ntiles) stage(nt % STAGES, nt * BK);
+        cp_async_commit();
+        const float* a = As + (t % STAGES) * SMEM_A + ty * AS_LD;
+        const float* b = Bs + (t % STAGES) * SMEM_B + tx * 4;
+        const int nk_tile = min(ksteps - t * BK, BK);
+#pragma unroll 1
+        for (int k0 = 0; k0 < nk_tile; k0 += 8) {
+            const int nk = min(nk_tile - k0, 8);
+            const bool again = t % 2 == 0 && k0 == 0;
+#pragma unroll
+            for (int i = 0; i < TM; i += R) {
+                float v[R][TN];
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) v[r][j] = ALGO == ALGO_TILE8 ? 0.0f : acc[i + r][j];
+                const float* ai = a + 16 * i * AS_LD + k0;
+                bool done = !never && (again || !(missed >> i & 1u));
+                if (done) done = short_steps<FMA, EIGHT, R, TN>(v, ai, 16 * AS_LD, b + k0 * BN, BN, nk, qa, qm);
+                missed &= ~(1u << i);
+                if (!done) {
+                    missed |= 1u << i;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        float4 e = ALGO == ALGO_TILE8 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(acc[i + r][0], acc[i + r][1], acc[i + r][2], acc[i + r][3]);
+#pragma unroll 1
+                        for (int k = 0; k < nk; ++k)
+                            e = mac_exact4<FMA>(e, a[16 * (i + r) * AS_LD + k0 + k], *reinterpret_cast<const float4*>(b + (k0 + k) * BN), pp);
+                        v[r][0] = e.x; v[r][1] = e.y; v[r][2] = e.z; v[r][3] = e.w;
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        if (ALGO != ALGO_TILE8) { acc[i + r][j] = v[r][j]; continue; }
+                        const float x = add_rn(outer[i + r][j], v[r][j]);
+                        Seen<EIGHT, true> seen;
+                        const float y = seen.round(qa, x);
+                        outer[i + r][j] = seen.covered(qa) ? y : exact_add_cold(pp, x);
+                    }
+            }
+        }
+    }
+    cp_async_wait<0>();
+    if (ALGO == ALGO_TILE8) store_tile<CONV_NONE>(p, C, m0, n0, ty, tx, p.vec != 0, outer);
+    else store_tile<CONV_NONE>(p, C, m0, n0, ty, tx, p.vec != 0, acc);
+}
+
+// As a call, for the sequential order's 128-row tiles: inlined it has their planned loop spill.
+template <int ALGO, bool FMA, bool EIGHT>
+__device__ __noinline__ void exact_tile16_call(const MmParams* pp) {
+    extern __shared__ __align__(16) float smem[];
+    int tile_m, tile_n;
+    banded_tile(tile_m, tile_n);
+    exact_tile16<ALGO, FMA, EIGHT>(pp, smem, blockIdx.z, tile_m * BM, tile_n * BN);
+}
+
 // ---- the kernel ------------------------------------------------------------------------------------------------------
 // Tiling, staging and epilogue are mm_kernel's: 128 x 64 outputs per CTA (64 x 64 in gemm16_mid.cu), 256 threads, 8 x 4
 // outputs per thread as 16 pairs, K slabs of 32 through three cp.async stages.
@@ -322,13 +467,26 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
 
     const FastPlan plan = make_plan<ALGO, FMA>(p, batch);
     if (CONV == CONV_NONE && p.defer_exact && !plan.ok) return;
+    // Where the second loop costs the planned one registers or time, entries without a plan redo group by group below: on the
+    // sequential order's 64-row tiles (768^3 in e8m7: 82 us with it, 72 without) and for fused sums on 128-row tiles in the CUDA
+    // order (96 x 1024 x 1024 x 64: 662 and 644).  Sums in e4m3, which hardly ever have a plan, always take it.
+    constexpr bool kPlanned = CONV == CONV_NONE && ALGO != ALGO_KAHAN && !NOSUB &&
+                              (SUM == SUM16_E4M3 || (ALGO == ALGO_TILE8 ? !(FMA && TM >= 8) : TM >= 8));
+    if constexpr (kPlanned) {         // from here on there is a plan
+        if (!plan.ok) {
+            if constexpr (ALGO == ALGO_SEQ && TM >= 8) exact_tile16_call<ALGO, FMA, SUM == SUM16_BF16>(&p);
+            else exact_tile16<ALGO, FMA, SUM == SUM16_BF16>(&p, smem, batch, m0, n0);
+            return;
+        }
+    }
+    const bool ok = kPlanned || plan.ok;
     // With a plan, the zero padding the CUDA order walks (and the last partial group of the sequential one, zero filled in
     // shared memory) adds zeros to add-format values, which changes none of them: whole groups, and only those with data.
     // Compensated sums do move under it (their compensation term is added), so they walk all of it.
     // Flushing sums can be -0, which + 0 turns into +0: the CUDA order's padding is walked too (it does that in the
     // reference), the sequential order's last partial group looks for -0 first.
     constexpr bool kFlush = NOSUB && sum_can_settle16(SUM, PROD);
-    const int ksteps = plan.ok && (ALGO == ALGO_SEQ || (ALGO == ALGO_TILE8 && !kFlush)) ? (p.K + 7) / 8 * 8
+    const int ksteps = ok && (ALGO == ALGO_SEQ || (ALGO == ALGO_TILE8 && !kFlush)) ? (p.K + 7) / 8 * 8
                      : (ALGO == ALGO_SEQ || (p.resume & MM_MORE)) ? p.K : p.K + 8 - p.K % 8;
     const int ntiles = (ksteps + BK - 1) / BK;
     const uint32_t lim = limit16<SUM>(plan.acc_limit), slab_lim = limit16<SUM>(plan.slab_limit);
@@ -400,8 +558,8 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
             const int nk = min(nk_tile - g * 8, 8);
             const bool wide = wide_start && t == 0 && g == 0;
             if (ALGO == ALGO_TILE8) {
-                bool redo = !plan.ok;
-                if (plan.ok) redo = group16<SUM, PROD, true, NOSUB>(acc, as, bs, g * 8, ty, tx, ns);
+                bool redo = !ok;
+                if (ok) redo = group16<SUM, PROD, true, NOSUB>(acc, as, bs, g * 8, ty, tx, ns);
                 if (redo) {
                     float f[TM][TN];
 #pragma unroll
@@ -413,7 +571,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
                 }
                 // fold the group into the outer sum
                 bool folded = false;
-                if (plan.ok && !wide && (slab_ok || all_below16<SUM>(aux, lim))) {
+                if (ok && !wide && (slab_ok || all_below16<SUM>(aux, lim))) {
                     uint32_t below = 0xFFFFFFFFu, out[TM][2];
 #pragma unroll
                     for (int i = 0; i < TM; ++i)
@@ -441,7 +599,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
             } else if (ALGO == ALGO_SEQ) {
                 bool redo = true;
                 const int kleft = p.K - t * BK - g * 8;
-                if (plan.ok && !wide && (slab_ok || all_below16<SUM>(acc, lim)) && !(kFlush && kleft < 8 && any_minus_zero16(acc))) {
+                if (ok && !wide && (slab_ok || all_below16<SUM>(acc, lim)) && !(kFlush && kleft < 8 && any_minus_zero16(acc))) {
                     uint32_t saved[TM][2];
                     if (kFlush) {
 #pragma unroll
@@ -460,7 +618,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mm16_kernel(const __grid_consta
                     pack_all16<SUM>(acc, f);
                 }
             } else {        // compensated sums; the reference pads K to a multiple of 8, so every group has 8 steps
-                if (plan.ok && all_below16<SUM>(acc, lim) && all_below16<SUM>(aux, lim)) {
+                if (ok && all_below16<SUM>(acc, lim) && all_below16<SUM>(aux, lim)) {
                     kahan_group16<SUM, PROD>(acc, aux, as, bs, g * 8, ty, tx);
                 } else {
                     float f[TM][TN], o[TM][TN];

@@ -24,9 +24,16 @@ __host__ __device__ constexpr int stagers(int conv) { return conv == CONV_WGRAD 
 __host__ __device__ constexpr int tb_ld(int conv) { return conv == CONV_WGRAD ? TBN + 2 : TBN + 4; }   // 4-byte column writes / 16-byte rows
 
 // `n` steps of a pair on the exact casters: a = the thread's row of the A slab, b = its column pair of the B slab.
-template <bool FMA>
+// SHORT: the short form first (entries without a plan in formats with subnormals).
+template <bool FMA, bool SHORT, bool EIGHT>
 __device__ __noinline__ float2 thin_exact_steps(float2 acc, const float* a, const float* b, int ldb, int n, const MmParams* pp) {
     const MmParams& p = *pp;
+    // a sum of an 8-bit-exponent format that continues from a -0 keeps its sign, which the short form does not
+    const bool minus_zero = __float_as_uint(acc.x) == 0x80000000u || __float_as_uint(acc.y) == 0x80000000u;
+    if (SHORT && !(EIGHT && minus_zero)) {
+        float v[1][2] = {{acc.x, acc.y}};
+        if (short_steps<FMA, EIGHT, 1, 2>(v, a, 0, b, ldb, n, ShortRn::make(p.wadd), ShortRn::make(p.wmul))) return make_float2(v[0][0], v[0][1]);
+    }
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
         const float av = a[k];
@@ -243,7 +250,7 @@ __global__ void __launch_bounds__(TTHREADS + stagers(CONV), CONV == CONV_WGRAD ?
             if (ALGO == ALGO_TILE8) {
                 bool redo = !plan.ok;
                 if (plan.ok) redo = thin_group16<SUM, PROD, true, NOSUB>(acc, ak, bk, LDB, ns);
-                if (redo) acc = pack16<SUM>(thin_exact_steps<FMA>(make_float2(0.0f, 0.0f), ak, bk, LDB, min(nk_tile - k0, 8), &p));
+                if (redo) acc = pack16<SUM>(thin_exact_steps<FMA, CONV == CONV_NONE && !NOSUB, SUM == SUM16_BF16>(make_float2(0.0f, 0.0f), ak, bk, LDB, min(nk_tile - k0, 8), &p));
                 bool folded = false;
                 if (plan.ok && !wide && pair_below16<SUM>(aux, lim)) {
                     uint32_t below = 0xFFFFFFFFu;
@@ -265,7 +272,7 @@ __global__ void __launch_bounds__(TTHREADS + stagers(CONV), CONV == CONV_WGRAD ?
                 const bool minus_zero = (acc & 0xFFFFu) == 0x8000u || (acc >> 16) == 0x8000u;
                 if (plan.ok && !wide && pair_below16<SUM>(acc, lim) && !(kFlush && kleft < 8 && minus_zero))
                     redo = thin_group16<SUM, PROD, false, NOSUB>(acc, ak, bk, LDB, ns);
-                if (redo) acc = pack16<SUM>(thin_exact_steps<FMA>(wide ? c_in : unpack16<SUM>(saved), ak, bk, LDB, min(min(nk_tile - k0, 8), kleft), &p));
+                if (redo) acc = pack16<SUM>(thin_exact_steps<FMA, CONV == CONV_NONE && !NOSUB, SUM == SUM16_BF16>(wide ? c_in : unpack16<SUM>(saved), ak, bk, LDB, min(min(nk_tile - k0, 8), kleft), &p));
             }
         }
     }
