@@ -46,9 +46,14 @@ KahanBounds kahan_bounds(int man) {
 }
 
 // Which tiles of the 16-bit kernel: 8 x 32 with one pair per thread (thin), 64 x 64 or 128 x 64?  A product takes the time of
-// the SM with the most tiles.  Measured for e4m3 products into e5m10 sums (clocks per K step and SM; the other formats scale
-// alike): n thin tiles 13 + 12 n, n tiles of 64 rows 122 n but never under 149, n of 128 rows 238 n.  256 x 256 x 4096: 94 us
-// thin, 310 and 490 otherwise; 768 x 768 x 1024: 140, 109, 156; 2048^2 x 512: 385, 239, 250.
+// the SM with the most tiles.  Measured for e4m3 products into e5m10 sums in the CUDA order (clocks per K step and SM): n thin
+// tiles 13 + 12 n, n tiles of 64 rows 122 n but never under 149, n of 128 rows 238 n.  256 x 256 x 4096: 94 us thin, 310 and
+// 490 otherwise; 768 x 768 x 1024: 140, 109, 156; 2048^2 x 512: 385, 239, 250.  Other forms have other clocks and one line
+// serves them all.  Squares x 1024 where its choice (*) misses the best tile by more than a tenth, us for 8, 64 and 128 rows:
+//   640   sequential e5m10 101* 78 128, sequential e8m7 95* 74 113, sequential and fused e5m10 99* 84 140
+//   768   e5m2 without subnormals 266 324* 634
+//   1024  e5m2 without subnormals 453 503 632*, sequential 517 472 560*
+//   1152  e5m2 without subnormals 564 672* 920;     1400  821 866 1018*
 enum Tile16 { TILE16_THIN, TILE16_MID, TILE16_BIG };
 Tile16 pick_tile16(int M, int N, int64_t batch, bool thin_allowed) {
     const int64_t sms = sm_count(), tn = ((int64_t)N + BN - 1) / BN;

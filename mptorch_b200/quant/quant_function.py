@@ -241,9 +241,11 @@ def quantizer(forward_number: Number | None = None, backward_number: Number | No
 def _mm_dispatch(a2, b2, batched, man_add, exp_add, man_mul, exp_mul, rounding, fma, subnormals, saturate,
                  compensated, rbits_add, rbits_mul):
     """One (possibly batched) GEMM on contiguous fp32 operands; allocates and returns C."""
-    # The kernel's CTA tile is 128 rows by 64 columns: a product with at most 64 rows and many columns would leave half of
+    # The FP32 kernel's CTA tile is 128 rows by 64 columns: a product with at most 64 rows and many columns would leave half of
     # every tile idle.  C^T = B^T A^T has the same products (multiplication commutes exactly) accumulated in the same
     # K order, so the transposed problem gives the same bits with full tiles; the result comes back as a transposed view.
+    # The kernels on 16-bit sums have tiles of 8 and 64 rows and gain nothing from it; they pay for the two copies
+    # (17 x 512 x 512: 45 us, called directly 24; 64 x 4096 x 4096: 300 and 215).
     # (Not for stochastic rounding: its random words are keyed by the position of the output in C.)
     if rounding == "nearest" and a2.shape[-2] <= 64 and b2.shape[-1] >= 256 and a2.shape[-1] >= 128:
         ct = _mm_dispatch(b2.transpose(-2, -1).contiguous(), a2.transpose(-2, -1).contiguous(), batched, man_add, exp_add, man_mul,
